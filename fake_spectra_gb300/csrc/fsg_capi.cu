@@ -669,10 +669,11 @@ DepositLaunch deposit_config(fsg_context *c, const LineParams &lp, const fsg_opt
     cfg.rec = tau32 && opt && opt->records == 1;
     if (opt && opt->records > 1)
         fail(FSG_ERR_VALUE, "records must be -1 (tuned), 0 or 1");
-    const int tdef = cfg.precision == FSG_PREC_FP64 ? 256 : 512;
+    cfg.fast64 = cfg.precision == FSG_PREC_FP64 && lp.compute_tau && !count;
+    const int tdef = cfg.precision == FSG_PREC_FP64 && !cfg.fast64 ? 256 : 512;
     const int tmax = cfg.precision == FSG_PREC_FP64 ? 256 : (tau32 ? 1024 : 512);
     cfg.threads = (opt && opt->threads > 0 && !vor) ? opt->threads : tdef;
-    if (cfg.threads % 32 || cfg.threads > tmax)
+    if (opt && opt->threads > 0 && !vor && (cfg.threads % 32 || cfg.threads > tmax))
         fail(FSG_ERR_VALUE, "threads must be a multiple of 32 and at most %d", tmax);
     cfg.tiles = cfg.tiles_asked = !(opt && opt->no_far_tiles);
     cfg.chunk = (opt && cfg.precision == FSG_PREC_FP32) ? opt->chunk : 0;
@@ -680,7 +681,8 @@ DepositLaunch deposit_config(fsg_context *c, const LineParams &lp, const fsg_opt
         fail(FSG_ERR_VALUE, "chunk must be between 1 and 32 (0 = tuned or default)");
     deposit_plan(cfg, lp.compute_tau, lp.nbins);
     cfg.persistent = (opt && opt->persistent >= 0 && !vor)
-                         ? opt->persistent : (cfg.precision == FSG_PREC_FP32 ? 1 : 0);
+                         ? opt->persistent
+                         : (cfg.precision == FSG_PREC_FP32 || cfg.fast64 ? 1 : 0);
     finish_config(c, lp, cfg);
     c->stats.launch_tuned = 0;
     return cfg;
@@ -796,6 +798,10 @@ fsg_tune_key tune_key(fsg_context *c, const LineParams &lp, int precision)
 void finish_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
 {
     int sms = 0;
+    if (cfg.fast64) {
+        deposit_clusters(cfg, lp.nbins, c->nlos);
+        return;
+    }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     const int per_sm = std::max(1, deposit_resident_ctas(cfg, lp.compute_tau, lp.nbins));
     cfg.grid = std::min(c->nlos, sms * per_sm);
@@ -1013,6 +1019,7 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
         put(cfgs[k].chunk);
         put(cfgs[k].tiles);
         put(cfgs[k].rec);
+        put(cfgs[k].cluster);
     }
     cudaStream_t s = c->own;
     cuda_check(cudaStreamSynchronize(c->stream), "sync caller stream");
@@ -1044,7 +1051,7 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
     cuda_check(cudaEventRecord(c->ev[2], s), "event");
     cuda_check(cudaGraphLaunch(c->graph, s), "graph launch");
     for (const DepositLaunch &cf : cfgs)   // deposit, fallback (+ tile weights)
-        c->stats.gpu_launches += 2 + (nlos > 0 && cf.tiles ? 1 : 0);
+        c->stats.gpu_launches += 2 + (nlos > 0 && cf.tiles && !cf.fast64 ? 1 : 0);
     cuda_check(cudaEventRecord(c->ev[3], s), "event");
     unsigned h_err = 0;
     cuda_check(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read");

@@ -1487,6 +1487,8 @@ __device__ __noinline__ void walk_tau_careful(const DepositArgs &a, const PairIn
     }
 }
 
+#include "fsg_tau64.cuh"
+
 // ------------------------------------------------------ far-field tiles
 // Far in a pair's damping wing (every pixel of a tile beyond the multipole
 // radius and at least TILE_DIST pixels from the line centre) the FP32 form
@@ -2660,10 +2662,39 @@ size_t stage_pair_bytes(int compute_tau, int precision)
 
 size_t deposit_smem_bytes(const DepositLaunch &cfg, int compute_tau, int nbins)
 {
+    if (cfg.fast64)
+        return (cfg.smem_mode ? (size_t)16 * nbins : 0) +
+               (size_t)16 * tiles64_layout(cfg.tiles, nbins).nodes +
+               (size_t)(cfg.threads / 32) * cfg.chunk * sizeof(Stage64);
     return (cfg.smem_mode ? (size_t)16 * nbins : 0) +
            (size_t)(cfg.threads / 32) * cfg.chunk * stage_pair_bytes(compute_tau, cfg.precision) +
            (cfg.tiles ? (size_t)16 * TILE_M * (nbins / TILE_W) : 0);
 }
+
+namespace {
+// FP64 optical depths through tau64_kernel.  The tile layout depends on nbins
+// only (room is kept for 16 warps of 4 staged pairs), so that every launch
+// sums the same values: the narrowest first tiles that fit, 64 pixels (up to
+// 8600 bins on GB300) to 256; accumulators go to global memory when they do
+// not fit beside the staged pairs.
+void plan_tau64(DepositLaunch &cfg, int nbins, size_t cap)
+{
+    const size_t stage_min = (size_t)(T64_THREADS / 32) * (T64_CHUNK / 2) * sizeof(Stage64);
+    const size_t acc = (size_t)16 * nbins;
+    const int asked = cfg.tiles;
+    cfg.fast64 = 1;
+    cfg.smem_mode = acc + stage_min <= cap;
+    cfg.tiles = 0;
+    if (asked)
+        for (int w0 = 64; w0 <= 256 && !cfg.tiles; w0 *= 2)
+            if ((cfg.smem_mode ? acc : 0) + stage_min +
+                    (size_t)16 * tiles64_layout(w0, nbins).nodes <= cap)
+                cfg.tiles = w0;
+    cfg.chunk = T64_CHUNK;
+    while (cfg.chunk > 1 && deposit_smem_bytes(cfg, 1, nbins) > cap)
+        cfg.chunk /= 2;
+}
+}  // namespace
 
 void deposit_plan(DepositLaunch &cfg, int compute_tau, int nbins)
 {
@@ -2701,6 +2732,10 @@ void deposit_plan(DepositLaunch &cfg, int compute_tau, int nbins)
         return;
     }
     cfg.chunk = 0;
+    if (compute_tau && cfg.fast64) {
+        plan_tau64(cfg, nbins, cap);
+        return;
+    }
     cfg.tiles = 0;
     cfg.smem_mode = (size_t)16 * nbins <= cap;
 }
@@ -2711,10 +2746,67 @@ int deposit_max_smem_bins(int compute_tau, int precision, int threads)
     return (int)(((size_t)(max_smem_optin() - STATIC_SMEM_RESERVE) - stage) / 16);
 }
 
+namespace {
+cudaLaunchConfig_t tau64_launch(int grid, int threads, size_t smem, int cluster,
+                                cudaLaunchAttribute *attr, cudaStream_t s)
+{
+    cudaFuncSetAttribute(tau64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((unsigned)grid);
+    lc.blockDim = dim3((unsigned)threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)cluster;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    return lc;
+}
+
+// Clusters of `cluster` tau64_kernel blocks that the device holds at once.
+int tau64_clusters(int threads, size_t smem, int cluster)
+{
+    cudaLaunchAttribute attr{};
+    const cudaLaunchConfig_t lc = tau64_launch(cluster, threads, smem, cluster, &attr, 0);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, tau64_kernel, &lc) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+}  // namespace
+
+// The cluster size with the least time for `nlos` equal sightlines, counting
+// whole waves: a wave of n clusters of c blocks takes 1/c of a sightline's
+// time, and each doubling costs a few percent (barriers, the shared sum).
+void deposit_clusters(DepositLaunch &cfg, int nbins, int nlos)
+{
+    const size_t smem = deposit_smem_bytes(cfg, 1, nbins);
+    double best = 1e300;
+    cfg.cluster = 1;
+    cfg.grid = nlos;
+    double penalty = 1.0;
+    for (int c = 1; c <= (cfg.smem_mode ? 8 : 1); c *= 2, penalty *= 1.04) {
+        const int n = tau64_clusters(cfg.threads, smem, c);
+        if (n <= 0)
+            continue;
+        const double t = penalty * std::ceil((double)nlos / n) / c;
+        if (t < best) {
+            best = t;
+            cfg.cluster = c;
+            cfg.grid = c * std::min(nlos, n);
+        }
+    }
+}
+
 int deposit_resident_ctas(const DepositLaunch &cfg, int compute_tau, int nbins)
 {
     const size_t smem = deposit_smem_bytes(cfg, compute_tau, nbins);
     const int threads = cfg.threads;
+    if (cfg.fast64)
+        return tau64_clusters(threads, smem, 1);
     if (compute_tau)
         return cfg.precision ? resident_ctas<true, 1, false>(threads, smem, cfg.rec != 0)
                              : resident_ctas<true, 0, false>(threads, smem, false);
@@ -2753,6 +2845,15 @@ int launch_deposit(const LineParams &lp, const LineTables &t, const Particles &p
         a.pl.rec = nullptr;
     const size_t smem = deposit_smem_bytes(cfg, lp.compute_tau, lp.nbins);
     int launched = 1;
+    if (cfg.fast64 && counters == nullptr) {
+        const int c = std::max(1, cfg.cluster);
+        cudaLaunchAttribute attr{};
+        const cudaLaunchConfig_t lc = tau64_launch(
+            cfg.persistent ? std::max(c, std::min(cfg.grid, c * nlos)) : c * nlos, cfg.threads,
+            smem, c, &attr, s);
+        cudaLaunchKernelEx(&lc, tau64_kernel, a);
+        return launched;
+    }
     if (cfg.tiles && counters == nullptr) {
         tile_weights_kernel<<<1, TILE_W * TILE_M, 0, s>>>();
         launched++;

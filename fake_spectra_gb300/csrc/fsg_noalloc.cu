@@ -303,12 +303,26 @@ int noalloc_run(int compute_tau, int nbins, int kernel, double box, double velfa
         cfg.precision = precision;
         cfg.threads = threads;
         cfg.tiles = 1;
-        deposit_plan(cfg, compute_tau, nbins);   // smem_mode = 1 within max_bins
-        cfg.persistent = precision == FSG_PREC_FP32 ? 1 : 0;
+        cfg.fast64 = precision == FSG_PREC_FP64 && compute_tau;
+        if (cfg.fast64) {
+            cfg.threads = 512;
+            deposit_plan(cfg, compute_tau, nbins);
+            if (!cfg.smem_mode) {   // no room beside the accumulators: the direct walk
+                cfg.fast64 = 0;
+                cfg.threads = threads;
+            }
+        }
+        if (!cfg.fast64)
+            deposit_plan(cfg, compute_tau, nbins);   // smem_mode = 1 within max_bins
+        cfg.persistent = precision == FSG_PREC_FP32 || cfg.fast64 ? 1 : 0;
         int sms = 0;
         NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
-        const int per_sm = std::max(1, deposit_resident_ctas(cfg, compute_tau, nbins));
-        cfg.grid = std::min(nlos, sms * per_sm);
+        if (cfg.fast64) {
+            deposit_clusters(cfg, nbins, nlos);
+        } else {
+            const int per_sm = std::max(1, deposit_resident_ctas(cfg, compute_tau, nbins));
+            cfg.grid = std::min(nlos, sms * per_sm);
+        }
         PairLists pl{d_off, d_part, d_dr2};
         NA_CUDA(cudaMemsetAsync(d_ticket, 0, 4, s), "memset");
         NA_CUDA(cudaMemsetAsync(d_nbad, 0, 4, s), "memset");
