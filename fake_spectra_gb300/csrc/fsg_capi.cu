@@ -799,7 +799,7 @@ void finish_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
 {
     int sms = 0;
     if (cfg.fast64) {
-        deposit_clusters(cfg, lp.nbins, c->nlos);
+        deposit_clusters(cfg, lp.compute_tau, lp.nbins, c->nlos);
         return;
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);

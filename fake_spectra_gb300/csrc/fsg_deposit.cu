@@ -34,6 +34,7 @@
 // propagate as they do in the reference.
 #include "fsg_internal.cuh"
 #include "fsg_voigt.cuh"
+#include "fsg_voigt_fix.cuh"
 
 #include <type_traits>
 
@@ -1334,7 +1335,9 @@ struct DepositArgs {
     int smem_mode;
     int persistent;
     int chunk;                      // pairs staged per warp (FP32 tau form)
-    int tiles;                      // far-field tile accumulators (FP32 tau form)
+    int tiles;                      // far-field tile accumulators (FP64 tau: the width of
+                                    // the narrowest tiles)
+    int table_off;                  // FP64 tau: byte offset of the staged K table, 0 = none
 };
 
 // FMT 0: 128-bit fixed point with carries (FP64 form); 1: split (FP32 form).
@@ -1488,6 +1491,7 @@ __device__ __noinline__ void walk_tau_careful(const DepositArgs &a, const PairIn
 }
 
 #include "fsg_tau64.cuh"
+#include "fsg_fast64.cuh"
 
 // ------------------------------------------------------ far-field tiles
 // Far in a pair's damping wing (every pixel of a tile beyond the multipole
@@ -2665,14 +2669,16 @@ size_t deposit_smem_bytes(const DepositLaunch &cfg, int compute_tau, int nbins)
     if (cfg.fast64)
         return (cfg.smem_mode ? (size_t)16 * nbins : 0) +
                (size_t)16 * tiles64_layout(cfg.tiles, nbins).nodes +
-               (size_t)(cfg.threads / 32) * cfg.chunk * sizeof(Stage64);
+               (size_t)(cfg.threads / 32) * cfg.chunk *
+                   sizeof(Stage64) +
+               (cfg.table ? sizeof(FixRow) * FSG_FIX_ROWS : 0);
     return (cfg.smem_mode ? (size_t)16 * nbins : 0) +
            (size_t)(cfg.threads / 32) * cfg.chunk * stage_pair_bytes(compute_tau, cfg.precision) +
            (cfg.tiles ? (size_t)16 * TILE_M * (nbins / TILE_W) : 0);
 }
 
 namespace {
-// FP64 optical depths through tau64_kernel.  The tile layout depends on nbins
+// FP64 optical depths through fast64_kernel.  The tile layout depends on nbins
 // only (room is kept for 16 warps of 4 staged pairs), so that every launch
 // sums the same values: the narrowest first tiles that fit, 64 pixels (up to
 // 8600 bins on GB300) to 256; accumulators go to global memory when they do
@@ -2690,8 +2696,12 @@ void plan_tau64(DepositLaunch &cfg, int nbins, size_t cap)
             if ((cfg.smem_mode ? acc : 0) + stage_min +
                     (size_t)16 * tiles64_layout(w0, nbins).nodes <= cap)
                 cfg.tiles = w0;
-    cfg.chunk = T64_CHUNK;
-    while (cfg.chunk > 1 && deposit_smem_bytes(cfg, 1, nbins) > cap)
+    // the K table (30 KB) in shared memory where 4 staged pairs still fit, else
+    // it is read through L1
+    cfg.chunk = T64_CHUNK / 2;
+    cfg.table = 1;
+    cfg.table = deposit_smem_bytes(cfg, 1, nbins) <= cap;
+    for (cfg.chunk = T64_CHUNK; cfg.chunk > 1 && deposit_smem_bytes(cfg, 1, nbins) > cap;)
         cfg.chunk /= 2;
 }
 }  // namespace
@@ -2732,7 +2742,7 @@ void deposit_plan(DepositLaunch &cfg, int compute_tau, int nbins)
         return;
     }
     cfg.chunk = 0;
-    if (compute_tau && cfg.fast64) {
+    if (cfg.fast64) {
         plan_tau64(cfg, nbins, cap);
         return;
     }
@@ -2747,10 +2757,17 @@ int deposit_max_smem_bins(int compute_tau, int precision, int threads)
 }
 
 namespace {
-cudaLaunchConfig_t tau64_launch(int grid, int threads, size_t smem, int cluster,
-                                cudaLaunchAttribute *attr, cudaStream_t s)
+decltype(&fast64_kernel<true>) fast64_build(int compute_tau)
 {
-    cudaFuncSetAttribute(tau64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    (void)compute_tau;
+    return fast64_kernel<true>;
+}
+
+cudaLaunchConfig_t fast64_launch(int compute_tau, int grid, int threads, size_t smem, int cluster,
+                                 cudaLaunchAttribute *attr, cudaStream_t s)
+{
+    cudaFuncSetAttribute(fast64_build(compute_tau), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3((unsigned)grid);
     lc.blockDim = dim3((unsigned)threads);
@@ -2764,13 +2781,14 @@ cudaLaunchConfig_t tau64_launch(int grid, int threads, size_t smem, int cluster,
     return lc;
 }
 
-// Clusters of `cluster` tau64_kernel blocks that the device holds at once.
-int tau64_clusters(int threads, size_t smem, int cluster)
+// Clusters of `cluster` fast64_kernel blocks that the device holds at once.
+int fast64_clusters(int compute_tau, int threads, size_t smem, int cluster)
 {
     cudaLaunchAttribute attr{};
-    const cudaLaunchConfig_t lc = tau64_launch(cluster, threads, smem, cluster, &attr, 0);
+    const cudaLaunchConfig_t lc = fast64_launch(compute_tau, cluster, threads, smem, cluster,
+                                                &attr, 0);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, tau64_kernel, &lc) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, fast64_build(compute_tau), &lc) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }
@@ -2781,15 +2799,15 @@ int tau64_clusters(int threads, size_t smem, int cluster)
 // The cluster size with the least time for `nlos` equal sightlines, counting
 // whole waves: a wave of n clusters of c blocks takes 1/c of a sightline's
 // time, and each doubling costs a few percent (barriers, the shared sum).
-void deposit_clusters(DepositLaunch &cfg, int nbins, int nlos)
+void deposit_clusters(DepositLaunch &cfg, int compute_tau, int nbins, int nlos)
 {
-    const size_t smem = deposit_smem_bytes(cfg, 1, nbins);
+    const size_t smem = deposit_smem_bytes(cfg, compute_tau, nbins);
     double best = 1e300;
     cfg.cluster = 1;
     cfg.grid = nlos;
     double penalty = 1.0;
     for (int c = 1; c <= (cfg.smem_mode ? 8 : 1); c *= 2, penalty *= 1.04) {
-        const int n = tau64_clusters(cfg.threads, smem, c);
+        const int n = fast64_clusters(compute_tau, cfg.threads, smem, c);
         if (n <= 0)
             continue;
         const double t = penalty * std::ceil((double)nlos / n) / c;
@@ -2806,7 +2824,7 @@ int deposit_resident_ctas(const DepositLaunch &cfg, int compute_tau, int nbins)
     const size_t smem = deposit_smem_bytes(cfg, compute_tau, nbins);
     const int threads = cfg.threads;
     if (cfg.fast64)
-        return tau64_clusters(threads, smem, 1);
+        return fast64_clusters(compute_tau, threads, smem, 1);
     if (compute_tau)
         return cfg.precision ? resident_ctas<true, 1, false>(threads, smem, cfg.rec != 0)
                              : resident_ctas<true, 0, false>(threads, smem, false);
@@ -2847,11 +2865,13 @@ int launch_deposit(const LineParams &lp, const LineTables &t, const Particles &p
     int launched = 1;
     if (cfg.fast64 && counters == nullptr) {
         const int c = std::max(1, cfg.cluster);
+        a.table_off = cfg.table ? (int)(smem - sizeof(FixRow) * FSG_FIX_ROWS) : 0;
         cudaLaunchAttribute attr{};
-        const cudaLaunchConfig_t lc = tau64_launch(
+        const cudaLaunchConfig_t lc = fast64_launch(
+            lp.compute_tau,
             cfg.persistent ? std::max(c, std::min(cfg.grid, c * nlos)) : c * nlos, cfg.threads,
             smem, c, &attr, s);
-        cudaLaunchKernelEx(&lc, tau64_kernel, a);
+        cudaLaunchKernelEx(&lc, fast64_build(lp.compute_tau), a);
         return launched;
     }
     if (cfg.tiles && counters == nullptr) {

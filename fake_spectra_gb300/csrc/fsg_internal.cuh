@@ -286,8 +286,9 @@ struct DepositLaunch {
                              // width of the narrowest tiles, 0 = none)
     int tiles_asked;         // what the caller allowed (tiles before planning)
     int rec;                 // FP32 tau: through pair records (PairLists::rec must be set)
-    int fast64;              // FP64 tau through tau64_kernel (planned with smem_mode)
-    int cluster;             // tau64_kernel: blocks that share a sightline
+    int fast64;              // FP64 through fast64_kernel (planned with smem_mode)
+    int table;               // fast64_kernel, tau: K table staged in shared memory
+    int cluster;             // fast64_kernel: blocks that share a sightline
 };
 
 // Deposits all pairs of all sightlines into out[L*nbins] (pre-zeroed).  Lines
@@ -306,8 +307,8 @@ int launch_deposit(const LineParams &lp, const LineTables &t, const Particles &p
 void deposit_plan(DepositLaunch &cfg, int compute_tau, int nbins);
 // Dynamic shared memory of one deposit CTA.
 size_t deposit_smem_bytes(const DepositLaunch &cfg, int compute_tau, int nbins);
-// tau64_kernel (cfg.fast64): blocks per cluster and the grid for nlos sightlines.
-void deposit_clusters(DepositLaunch &cfg, int nbins, int nlos);
+// fast64_kernel (cfg.fast64): blocks per cluster and the grid for nlos sightlines.
+void deposit_clusters(DepositLaunch &cfg, int compute_tau, int nbins, int nlos);
 // CTAs of the deposit kernel that fit on one SM for this configuration.
 int deposit_resident_ctas(const DepositLaunch &cfg, int compute_tau, int nbins);
 // Plain FP64 atomics into out for the listed lines (non-finite propagation).

@@ -318,7 +318,7 @@ int noalloc_run(int compute_tau, int nbins, int kernel, double box, double velfa
         int sms = 0;
         NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
         if (cfg.fast64) {
-            deposit_clusters(cfg, nbins, nlos);
+            deposit_clusters(cfg, compute_tau, nbins, nlos);
         } else {
             const int per_sm = std::max(1, deposit_resident_ctas(cfg, compute_tau, nbins));
             cfg.grid = std::min(nlos, sms * per_sm);

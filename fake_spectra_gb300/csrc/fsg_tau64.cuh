@@ -32,10 +32,14 @@
 //    distributed shared memory at the end (integer sums: the same bits for
 //    every cluster size).
 //
-// Measured (GB300, device time): 72 sightlines x 6691 pixels of a 256^3
-// snapshot 1632 ms with the direct walk, 255 ms so; 400 sightlines x 1115
-// pixels of 128^3, CIV (little wing) 911 and 588 ms.  The 7 profiles of the
-// pixels inside vmp bound it (FP64 pipe).
+//  * Inside vmp the 7 profiles are summed in 64-bit integers
+//    (fsg_voigt_fix.cuh), whose instructions issue 16 to 64 times as fast as
+//    FP64 ones.
+//
+// Measured (GB300, whole call): 72 sightlines x 6691 pixels of a 256^3
+// snapshot 1766 ms with the direct walk, 255 ms with FP64 profiles inside vmp,
+// 20.5 ms so; 400 sightlines x 1115 pixels of 128^3, CIV (little wing) 1028,
+// 588 and 26.8 ms.
 //
 // Pairs outside the series' conditions (a <= 0 or a > 0.1, non-finite
 // constants, a pixel width within 1e-9 of a sub-sampling boundary) take the
@@ -50,15 +54,20 @@ constexpr int T64_THREADS = 512;
 constexpr int T64_CHUNK = 8;
 
 constexpr int S64_SKIP = 1 << 30, S64_CAREFUL = 1 << 29, S64_TILES = 1 << 28;
-constexpr int S64_NP = (1 << 28) - 1;
+constexpr int S64_FIX = 1 << 27;         // node sums in integers (fsg_voigt_fix.cuh)
+constexpr int S64_NP = (1 << 27) - 1;
 
 struct __align__(16) Stage64 {
     double vel, zd;          // particle velocity; its pixel zmax as a double
-    double inv_b, aa;
+    double inv_b, inv_lo;    // 1/b as a sum of two doubles
+    double aa, vmp;
     double scale;            // amp dens / velfac x node spacing / (npoints - 1)
     double u1;               // node spacing / b: node i at (i - 3) u1
-    double vmp;
-    double w[NODES];         // kernel weights
+    double cg, ck;           // S64_FIX: factors of the two integer sums
+    union {
+        double w[NODES];     // kernel weights
+        FixPair fix;
+    };
     double A[T64_R];         // far-wing coefficients times vmp^(-2r)
     float vsure;             // tiles out to this |V| hold no pixel below tautail
     int j0, flags, pad;
@@ -132,7 +141,7 @@ __device__ __forceinline__ bool stage64_setup(const LineParams &lp, const PairIn
     Tau64 s;
     if (!s.setup(lp, in))
         return false;
-    const double u1 = s.deltav * s.inv_b;
+    const double u1 = s.deltav * s.inv_b, vk = s.bintov * s.inv_b;
     const double umax = 3.0 * fabs(u1);
     const double vmp = fmax(4.5 * umax, umax + 12.0);
     // tau_kern_outer sub-samples (singleabs.h:104-126): uniform over the pair
@@ -157,12 +166,35 @@ __device__ __forceinline__ bool stage64_setup(const LineParams &lp, const PairIn
     st.scale = sc;
     st.u1 = u1;
     st.vmp = vmp;
-#pragma unroll
-    for (int i = 0; i < NODES; i++)
-        st.w[i] = s.w[i];
+    st.inv_lo = fma(-s.inv_b, s.btherm, 1.0) * s.inv_b;
     st.j0 = s.bin0(lp.nbins);
     bool tiles = false;
     float vsure = 0.f;
+    // the integer node sums: V within their range for every pixel step that
+    // reaches inside vmp (one step of 32 pixels and its outer edge beyond it)
+    double wmax = 0.0;
+#pragma unroll
+    for (int i = 0; i < NODES; i++)
+        wmax = fmax(wmax, s.w[i]);
+    const bool fix = !careful && s.aa >= FIXV_A_MIN && s.aa <= FIXV_A_MAX && wmax > 0.0 &&
+                     fabs(sc) * wmax > 1e-200 && vmp + umax + 34.0 * vk < FIXV_MAX;
+    if (fix) {
+        const double inv_w = 1.0 / wmax;
+        fix_pair_damping(s.aa, st.fix);
+        st.fix.u1 = __double2ll_rn(u1 * 9007199254740992.0);
+#pragma unroll
+        for (int i = 0; i < NODES; i++) {
+            const double q = s.w[i] * inv_w * 4611686018427387904.0;   // 2^62
+            st.fix.w[i] = fix62(min(__double2ull_rn(q), (1ull << 62) - 1ull) << 2);
+        }
+        const double c = sc * wmax * 8.673617379884035e-19;            // 2^-60
+        st.cg = c * exp(s.aa * s.aa);
+        st.ck = c * s.aa;
+    } else {
+#pragma unroll
+        for (int i = 0; i < NODES; i++)
+            st.w[i] = s.w[i];
+    }
     if (!careful) {
         far_coefficients64(s.w, u1, s.aa, vmp, st.A);
         tiles = sc > 0.0 && st.A[0] > 0.0;
@@ -200,7 +232,8 @@ __device__ __forceinline__ bool stage64_setup(const LineParams &lp, const PairIn
         }
     }
     st.vsure = vsure;
-    st.flags = np | (careful ? S64_CAREFUL : 0) | (tiles ? S64_TILES : 0);
+    st.flags = np | (careful ? S64_CAREFUL : 0) | (tiles ? S64_TILES : 0) |
+               (fix ? S64_FIX : 0);
     st.pad = 0;
     return true;
 }
@@ -227,9 +260,42 @@ __host__ __device__ inline Tiles64 tiles64_layout(int w0, int nbins)
 // cos(pi j / 32), j = 0 .. 63 (Chebyshev nodes and their transform)
 __shared__ double s_cos64[64];
 
-// A pair's node sum times scale at V (all lanes call it).
-__device__ __forceinline__ double inner64(const Stage64 &st, double V)
+// K table rows: in shared memory the 16-byte words of row r are exchanged by
+// the bits of r / 2, so that 8 lanes reading the same word of different rows
+// spread over all banks.
+struct Rows64 {
+    const FixRow *rows;
+    int mask;                // 3 in shared memory, 0 in global memory
+    __device__ __forceinline__ FixRow load(int r) const
+    {
+        const char *p = reinterpret_cast<const char *>(rows + r);
+        const int sw = ((r >> 1) & mask) << 4;
+        union {
+            int4 q[4];
+            FixRow row;
+        } u;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            u.q[i] = *reinterpret_cast<const int4 *>(p + ((i << 4) ^ sw));
+        return u.row;
+    }
+};
+
+__device__ const FixRow d_fix_rows[FSG_FIX_ROWS] = FSG_FIX_INIT;
+__device__ const Fix62 d_fix_pow2[64] = FSG_FIX_POW2_INIT;
+__shared__ Fix62 s_pow2[64];
+
+// d 2^-e (e >= 0) of a normal d that stays normal
+__device__ __forceinline__ double exp_down(double d, int e)
 {
+    return __hiloint2double(__double2hiint(d) - (e << 20), __double2loint(d));
+}
+
+// A pair's node sum times scale at velocity v from the line centre (all lanes
+// call it).
+__device__ __forceinline__ double inner64(const Stage64 &st, const Rows64 &rows, double v)
+{
+    const double V = v * st.inv_b;
     const double av = fabs(V);
     const double vmp = st.vmp;
     if (__all_sync(0xffffffffu, av >= vmp)) {
@@ -254,6 +320,17 @@ __device__ __forceinline__ double inner64(const Stage64 &st, double V)
         }
         return st.scale * (s * y);
     }
+    if (st.flags & S64_FIX) {
+        // V to 2^-53: the product's rounding error is added back
+        const double lo = fma(v, st.inv_lo, fma(v, st.inv_b, -V));
+        const int64_t vi = __double2ll_rn(V * 9007199254740992.0) +
+                           __double2ll_rn(lo * 9007199254740992.0);
+        int64_t sg, sk;
+        int eg, ek;
+        fix_node_sums(st.fix, vi, rows, s_pow2, sg, eg, sk, ek);
+        return fma(exp_down(st.cg, eg), __ll2double_rn(sg),
+                   exp_down(st.ck, ek) * __ll2double_rn(sk));
+    }
     const double aa = st.aa, u1 = st.u1;
     double total = 0.0;
 #pragma unroll 1
@@ -264,18 +341,19 @@ __device__ __forceinline__ double inner64(const Stage64 &st, double V)
 
 // The pair's optical depth at a low pixel edge vlow (velocity from the line
 // centre), tau_kern_outer's rule.
-__device__ __forceinline__ double outer64(const Stage64 &st, double vlow, double bintov)
+__device__ __forceinline__ double outer64(const Stage64 &st, const Rows64 &rows, double vlow,
+                                          double bintov)
 {
     const double vhigh = __dadd_rn(vlow, bintov);
     const int np = st.flags & S64_NP;
     if (np == 1)
-        return inner64(st, __dmul_rn(0.5, __dadd_rn(vhigh, vlow)) * st.inv_b);
+        return inner64(st, rows, __dmul_rn(0.5, __dadd_rn(vhigh, vlow)));
     const double dv = (vhigh - vlow) / (np - 1);
     double total = 0.0;
 #pragma unroll 1
     for (int i = 0; i < np; i++) {
         const double v = i == np - 1 ? vhigh : __dadd_rn(__dmul_rn((double)i, dv), vlow);
-        const double f = inner64(st, v * st.inv_b);
+        const double f = inner64(st, rows, v);
         total = (i == 0 || i == np - 1) ? fma(0.5, f, total) : total + f;
     }
     return total;
@@ -297,7 +375,8 @@ __device__ __noinline__ void walk64_careful(const DepositArgs &a, const PairInpu
 // k = c - c0 counts pixels from the line centre, and c0 drops by nbins where
 // the window wraps.  Tiles start where c is a multiple of their width.
 __device__ __forceinline__ void walk_tau64(const DepositArgs &a, const Tiles64 &tl,
-                                           const Stage64 &st, int S, unsigned long long *lo,
+                                           const Rows64 &rows, const Stage64 &st, int S,
+                                           unsigned long long *lo,
                                            unsigned long long *hi, unsigned long long *tlo,
                                            unsigned long long *thi, int *bad, int lane,
                                            double bintov)
@@ -390,7 +469,7 @@ __device__ __forceinline__ void walk_tau64(const DepositArgs &a, const Tiles64 &
                         const int kt = ct - c0;
                         const double off = (double)(dir == 0 ? kt : -kt - w) + x;
                         const double vlow = fma(off, bintov, fma(zd, bintov, -vel));
-                        const double v = outer64(st, vlow, bintov);
+                        const double v = outer64(st, rows, vlow, bintov);
                         if (on) {
                             const int tile = dir == 0 ? ct / w : -(ct / w) - 1;
                             const int first = l == 0 ? tl.first[0]
@@ -408,7 +487,7 @@ __device__ __forceinline__ void walk_tau64(const DepositArgs &a, const Tiles64 &
             len = min(len, limit - c);
             const int koff = dir == 0 ? k + lane : -1 - k - lane;
             const double vlow = __dsub_rn(__dmul_rn(zd + (double)koff, bintov), vel);
-            const double v = outer64(st, vlow, bintov);
+            const double v = outer64(st, rows, vlow, bintov);
             const bool valid = lane < len && k + lane < half;
             const unsigned m = __ballot_sync(0xffffffffu, valid && v < tautail);
             const int last = m ? (__ffs(m) - 1) : 31;
@@ -422,242 +501,30 @@ __device__ __forceinline__ void walk_tau64(const DepositArgs &a, const Tiles64 &
     }
 }
 
-__device__ __forceinline__ unsigned cluster_size()
+// One chunk of pairs [cb, cb + n) of a sightline, whole warp.
+__device__ __forceinline__ void deposit_tau64(const DepositArgs &a, const Tiles64 &tl,
+                                              const Rows64 &rows, int axis, long long cb, int n,
+                                              int S, unsigned long long *lo,
+                                              unsigned long long *hi, unsigned long long *tlo,
+                                              unsigned long long *thi, int *bad, Stage64 *stage,
+                                              double bintov, int lane)
 {
-    unsigned n;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
-    return n;
-}
-__device__ __forceinline__ unsigned cluster_rank()
-{
-    unsigned r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// Barrier of every thread of the cluster (release / acquire).
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The address of this block's shared object in the block of rank r.
-template <class T>
-__device__ __forceinline__ T *cluster_map(T *p, unsigned r)
-{
-    unsigned long long out;
-    asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"((unsigned long long)p), "r"(r));
-    return reinterpret_cast<T *>(out);
-}
-
-// Sum over the cluster's blocks of a 128-bit accumulator word, as a double.
-__device__ __forceinline__ double cluster_fixed(unsigned long long *lo, unsigned long long *hi,
-                                                unsigned nc, int S)
-{
-    unsigned long long l = lo[0], h = hi[0];
-    if (nc > 1) {
-        l = 0ull;
-        h = 0ull;
-        for (unsigned r = 0; r < nc; r++) {
-            const unsigned long long x = *cluster_map(lo, r);
-            h += *cluster_map(hi, r);
-            l += x;
-            h += l < x ? 1ull : 0ull;
-        }
+    if (lane < n) {
+        const PairInput in = load_pair(a.p, a.pl, cb + lane, axis, true, a.dev_err);
+        if (!stage64_setup(a.lp, in, stage[lane]))
+            stage[lane].flags = S64_SKIP;
     }
-    return from_fixed(l, h, S);
-}
-
-// Clenshaw sum of the M Chebyshev coefficients c at t in [-1, 1].
-__device__ __forceinline__ double clenshaw64(const double *c, double t)
-{
-    double b1 = 0.0, b2 = 0.0;
-    const double t2 = 2.0 * t;
-#pragma unroll
-    for (int k = T64_M - 1; k >= 1; k--) {
-        const double b = fma(t2, b1, c[k] - b2);
-        b2 = b1;
-        b1 = b;
+    __syncwarp();
+    for (int q = 0; q < n; q++) {
+        const Stage64 &st = stage[q];
+        if (st.flags & S64_SKIP)
+            continue;
+        if (st.flags & S64_CAREFUL) {
+            const PairInput in = load_pair(a.p, a.pl, cb + q, axis, true, a.dev_err);
+            walk64_careful(a, in, S, lo, hi, bad, lane);
+            continue;
+        }
+        walk_tau64(a, tl, rows, st, S, lo, hi, tlo, thi, bad, lane, bintov);
     }
-    return fma(t, b1, c[0] - b2);
-}
-
-// Node values of `ntiles` tiles to Chebyshev coefficients, in place (half a
-// warp per tile, whole block).
-__device__ __forceinline__ void nodes_to_coefs64(double *node, int ntiles)
-{
-    static_assert(T64_M == 16, "half a warp per tile; s_cos64 has 64 entries");
-    const int k = threadIdx.x & 15;
-    const int per = blockDim.x / 16;
-    for (int t0 = 0; t0 < ntiles; t0 += per) {
-        const int t = t0 + threadIdx.x / 16;
-        double *f = node + (size_t)t * T64_M;
-        double s = 0.0;
-        if (t < ntiles) {
-#pragma unroll
-            for (int m = 0; m < T64_M; m++)
-                s = fma(f[m], s_cos64[(k * (2 * m + 1)) & 63], s);
-            s *= k == 0 ? 1.0 / T64_M : 2.0 / T64_M;
-        }
-        __syncwarp();
-        if (t < ntiles)
-            f[k] = s;
-        __syncwarp();
-    }
-}
-
-__global__ void __launch_bounds__(T64_THREADS, 1) tau64_kernel(DepositArgs a)
-{
-    extern __shared__ __align__(16) unsigned long long smem[];
-    __shared__ BoundScratch red;
-    __shared__ int s_bad;
-    __shared__ unsigned s_ticket, s_chunk;
-    const int nbins = a.lp.nbins;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned nc = cluster_size(), rank = cluster_rank();
-    const double bintov = a.lp.vbox / nbins;
-    const Tiles64 tl = tiles64_layout(a.tiles, nbins);
-    // dynamic shared memory: [accumulators lo, hi (smem_mode)] [tile nodes lo, hi] [stage]
-    unsigned long long *tlo = smem + (a.smem_mode ? 2 * (size_t)nbins : 0);
-    unsigned long long *thi = tlo + tl.nodes;
-    Stage64 *stage = reinterpret_cast<Stage64 *>(smem + (a.smem_mode ? 2 * (size_t)nbins : 0) +
-                                                 2 * (size_t)tl.nodes) + warp * a.chunk;
-    for (int j = threadIdx.x; j < 64; j += blockDim.x)
-        s_cos64[j] = cospi((double)j / 32.0);
-    const unsigned first = blockIdx.x / nc;
-    unsigned ticket = first;
-    for (;;) {
-        if (a.persistent) {
-            // the cluster's first block draws the next sightline
-            if (rank == 0 && threadIdx.x == 0) {
-                const unsigned t = atomicAdd(a.ticket, 1u);
-                for (unsigned r = 0; r < nc; r++)
-                    *cluster_map(&s_ticket, r) = t;
-            }
-            cluster_sync();
-            ticket = s_ticket;
-        }
-        if (ticket >= (unsigned)a.nlos)
-            break;
-        const int line = a.line_order[ticket];
-        const int axis = a.t.axis[line];
-        const long long e0 = a.pl.off[line], e1 = a.pl.off[line + 1];
-        const double B = order_free_bound(
-            e0, e1,
-            [&](long long e) {
-                return tau_pair_bound(a.lp, load_pair(a.p, a.pl, e, axis, true, a.dev_err));
-            },
-            [&](long long e) {
-                return tau_pair_bound(a.lp, load_pair(a.p, a.pl, e, axis, true, a.dev_err));
-            },
-            &red);
-        unsigned long long *lo, *hi;
-        if (a.smem_mode) {
-            lo = smem;
-            hi = smem + nbins;
-        } else {
-            lo = a.gacc + (size_t)line * 2 * nbins;
-            hi = lo + nbins;
-        }
-        for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
-            lo[j] = 0ull;
-            hi[j] = 0ull;
-        }
-        for (int j = threadIdx.x; j < tl.nodes; j += blockDim.x) {
-            tlo[j] = 0ull;
-            thi[j] = 0ull;
-        }
-        if (threadIdx.x == 0) {
-            s_chunk = 0u;
-            s_bad = !isfinite(B);
-        }
-        cluster_sync();
-        const bool live = isfinite(B) && B > 0.0;
-        const int S = live ? 124 - ilogb(B) : 0;
-        if (live) {
-            unsigned *counter = cluster_map(&s_chunk, 0);
-            for (;;) {
-                unsigned c = 0;
-                if (lane == 0)
-                    c = atomicAdd(counter, 1u);
-                c = __shfl_sync(0xffffffffu, c, 0);
-                const long long cb = e0 + (long long)c * a.chunk;
-                if (cb >= e1)
-                    break;
-                const int n = (int)min((long long)a.chunk, e1 - cb);
-                if (lane < n) {
-                    const PairInput in = load_pair(a.p, a.pl, cb + lane, axis, true, a.dev_err);
-                    if (!stage64_setup(a.lp, in, stage[lane]))
-                        stage[lane].flags = S64_SKIP;
-                }
-                __syncwarp();
-                for (int q = 0; q < n; q++) {
-                    const Stage64 &st = stage[q];
-                    if (st.flags & S64_SKIP)
-                        continue;
-                    if (st.flags & S64_CAREFUL) {
-                        const PairInput in = load_pair(a.p, a.pl, cb + q, axis, true, a.dev_err);
-                        walk64_careful(a, in, S, lo, hi, &s_bad, lane);
-                        continue;
-                    }
-                    walk_tau64(a, tl, st, S, lo, hi, tlo, thi, &s_bad, lane, bintov);
-                }
-                __syncwarp();
-            }
-        }
-        cluster_sync();
-        bool bad = s_bad != 0;
-        for (unsigned r = 0; r < nc && !bad; r++)
-            bad = *cluster_map(&s_bad, r) != 0;
-        if (bad) {
-            if (rank == 0 && threadIdx.x == 0)
-                a.bad_lines[atomicAdd(a.n_bad, 1)] = line;
-        } else if (live) {
-            double *row = a.out + (size_t)line * nbins;
-            double *node = reinterpret_cast<double *>(tlo);
-            if (tl.nodes > 0) {
-                // node sums as doubles: each block forms its share for all blocks
-                for (int j = rank * blockDim.x + threadIdx.x; j < tl.nodes;
-                     j += nc * blockDim.x) {
-                    const double v = cluster_fixed(tlo + j, thi + j, nc, S);
-                    if (nc == 1)
-                        node[j] = v;
-                    else
-                        for (unsigned r = 0; r < nc; r++)
-                            *cluster_map(node + j, r) = v;
-                }
-                cluster_sync();
-                // from the widest tiles down: coefficients, added at the nodes
-                // of the four tiles below
-                for (int l = T64_LEVELS - 1; l >= 0; l--) {
-                    const int nt = nbins / (tl.w0 << (2 * l));
-                    double *nd = node + tl.first[l];
-                    nodes_to_coefs64(nd, nt);
-                    __syncthreads();
-                    if (l > 0) {
-                        double *down = node + tl.first[l - 1];
-                        for (int j = threadIdx.x; j < nt * 4 * T64_M; j += blockDim.x) {
-                            const int child = j / T64_M, m = j % T64_M;
-                            const double t = fma(0.25, s_cos64[2 * m + 1],
-                                                 0.5 * (double)(child & 3) - 0.75);
-                            down[j] += clenshaw64(nd + (size_t)(child >> 2) * T64_M, t);
-                        }
-                        __syncthreads();
-                    }
-                }
-            }
-            const int covered = tl.w0 > 0 ? nbins / tl.w0 * tl.w0 : 0;
-            const double inv_w = tl.w0 > 0 ? 2.0 / tl.w0 : 0.0;
-            for (int j = rank * blockDim.x + threadIdx.x; j < nbins; j += nc * blockDim.x) {
-                double v = cluster_fixed(lo + j, hi + j, nc, S);
-                if (j < covered)
-                    v += clenshaw64(node + (size_t)(j / tl.w0) * T64_M,
-                                    fma((double)(j & (tl.w0 - 1)) + 0.5, inv_w, -1.0));
-                row[j] = v;
-            }
-        }
-        // no block clears or leaves its accumulators while another reads them
-        cluster_sync();
-        if (!a.persistent)
-            break;
-    }
+    __syncwarp();
 }
