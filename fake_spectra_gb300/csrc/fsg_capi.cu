@@ -669,7 +669,7 @@ DepositLaunch deposit_config(fsg_context *c, const LineParams &lp, const fsg_opt
     cfg.rec = tau32 && opt && opt->records == 1;
     if (opt && opt->records > 1)
         fail(FSG_ERR_VALUE, "records must be -1 (tuned), 0 or 1");
-    cfg.fast64 = cfg.precision == FSG_PREC_FP64 && lp.compute_tau && !count;
+    cfg.fast64 = cfg.precision == FSG_PREC_FP64 && !count;
     const int tdef = cfg.precision == FSG_PREC_FP64 && !cfg.fast64 ? 256 : 512;
     const int tmax = cfg.precision == FSG_PREC_FP64 ? 256 : (tau32 ? 1024 : 512);
     cfg.threads = (opt && opt->threads > 0 && !vor) ? opt->threads : tdef;

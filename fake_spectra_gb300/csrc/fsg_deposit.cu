@@ -35,6 +35,7 @@
 #include "fsg_internal.cuh"
 #include "fsg_voigt.cuh"
 #include "fsg_voigt_fix.cuh"
+#include "fsg_spline_fix.cuh"
 
 #include <type_traits>
 
@@ -1491,6 +1492,7 @@ __device__ __noinline__ void walk_tau_careful(const DepositArgs &a, const PairIn
 }
 
 #include "fsg_tau64.cuh"
+#include "fsg_colden64.cuh"
 #include "fsg_fast64.cuh"
 
 // ------------------------------------------------------ far-field tiles
@@ -2142,6 +2144,10 @@ __global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(
     unsigned long long *acc = a.smem_mode ? smem : a.gacc + (size_t)blockIdx.x * acc_words;
     StageColK *sw = reinterpret_cast<StageColK *>(smem + (a.smem_mode ? acc_words : 0)) +
                     warp * a.chunk;
+    // FP64: the staged geometry, after every warp's StageColK rows
+    StageC64 *sw64 = reinterpret_cast<StageC64 *>(
+                         reinterpret_cast<StageColK *>(smem + (a.smem_mode ? acc_words : 0)) +
+                         (blockDim.x >> 5) * a.chunk) + warp * a.chunk;
     if (threadIdx.x == 0)
         s_ticket = atomicAdd(a.ticket, 1u);
     __syncthreads();
@@ -2190,7 +2196,15 @@ __global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(
                 StageColK st;
                 Colden col;
                 st.flags = 0;
-                if (!col.setup(a.lp, in, btk)) {
+                if constexpr (PREC == 0) {
+                    bool ok;
+                    stagec64_setup(a.lp, in, btk, sw64[lane], ok);
+                    if (!ok) {
+                        atomicOr(a.dev_err, (unsigned)DEVERR_WINDOW_LIMIT);
+                        for (int c = 0; c < nch; c++)
+                            s_bad[c] = 1;
+                    }
+                } else if (!col.setup(a.lp, in, btk)) {
                     st.flags = COL_SKIP;
                 } else if (!col.ok) {
                     st.flags = COL_BAD;
@@ -2202,16 +2216,14 @@ __global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(
                         return kern_frac<double>(a.lp.kernel, plow, __dadd_rn(plow, btk), col.smooth,
                                                  col.dr2, col.zrange);
                     };
-                    if constexpr (PREC == 1) {
-                        st.kf0 = kf(col.zlow);
-                        st.kf1 = col.kmax >= 2 ? kf(col.zlow + col.kmax - 1) : 0.0;
-                        st.kf2 = col.kmax >= 1 ? kf(col.zhigh) : 0.0;
-                        st.dL0 = col.dL0;
-                        st.dR0 = col.dR0;
-                        st.two_zr = col.two_zr;
-                        st.inv_h2 = col.inv_h2;
-                        st.ch = col.ch;
-                    }
+                    st.kf0 = kf(col.zlow);
+                    st.kf1 = col.kmax >= 2 ? kf(col.zlow + col.kmax - 1) : 0.0;
+                    st.kf2 = col.kmax >= 1 ? kf(col.zhigh) : 0.0;
+                    st.dL0 = col.dL0;
+                    st.dR0 = col.dR0;
+                    st.two_zr = col.two_zr;
+                    st.inv_h2 = col.inv_h2;
+                    st.ch = col.ch;
                 }
                 const int ip = a.pl.part[cb + lane];
 #pragma unroll
@@ -2222,7 +2234,26 @@ __global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(
                 sw[lane] = st;
             }
             __syncwarp();
-            for (int k2 = 0; k2 < n; k2++) {
+            if constexpr (PREC == 0) {
+                // the pixels and values of deposit_colden64, times each channel's density
+                const auto put = [&](int p, int k2, double f) {
+                    const int j = col_bin(sw64[p].j0, k2, nbins);
+#pragma unroll
+                    for (int c = 0; c < MAX_CHANNELS; c++)
+                        if (live[c])
+                            accumulate<double, 0>(a.dev_err, __dmul_rn((double)sw[p].dens[c], f),
+                                                  j, S[c], acc + 2 * (size_t)c * nbins,
+                                                  acc + (2 * (size_t)c + 1) * nbins, &s_bad[c]);
+                };
+                for (int q2 = 0; q2 < n; q2++)
+                    for (int k2 = sw64[q2].ilo + lane; k2 <= sw64[q2].ihi; k2 += 32)
+                        put(q2, k2, colden64_interior(sw64[q2], a.lp.kernel, btk, k2));
+                for_each_edge64(sw64, n, lane, [&](int p, int k2) {
+                    put(p, k2, colden64_direct(sw64[p], a.lp.kernel, btk, k2));
+                });
+                __syncwarp();
+            }
+            for (int k2 = 0; PREC == 1 && k2 < n; k2++) {
                 const StageColK st = sw[k2];
                 if (st.flags == COL_SKIP)
                     continue;
@@ -2233,55 +2264,35 @@ __global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(
                         s_bad[c] = 1;
                     continue;
                 }
-                // the FP64 form needs the pair's geometry again: rebuild it from the pair
-                Colden col;
-                if constexpr (PREC == 0) {
-                    const PairInput in = load_pair_ch(a, cb + k2, axis, 0);
-                    col.setup(a.lp, in, btk);
-                }
                 int j = st.j0 + lane;
                 while (j >= nbins)
                     j -= nbins;
                 for (int k = lane; k <= st.kmax; k += 32) {
-                    if constexpr (PREC == 0) {
-                        const double plow = __dsub_rn(__dmul_rn(btk, (double)(col.zlow + k)),
-                                                      col.pos1);
-                        const double f = kern_frac<double>(a.lp.kernel, plow, __dadd_rn(plow, btk),
-                                                           col.smooth, col.dr2, col.zrange);
-#pragma unroll
-                        for (int c = 0; c < MAX_CHANNELS; c++)
-                            if (live[c])
-                                accumulate<double, 0>(a.dev_err, (double)st.dens[c] * f, j, S[c],
-                                                      acc + 2 * (size_t)c * nbins,
-                                                      acc + (2 * (size_t)c + 1) * nbins,
-                                                      &s_bad[c]);
-                    } else {
-                        const bool edge = k == 0 || k >= st.kmax - 1;
-                        const double fe = k == 0 ? st.kf0 : (k == st.kmax ? st.kf2 : st.kf1);
-                        float f32 = 0.f;
-                        if (!edge) {
-                            StageCol32 g;
-                            g.kmax = st.kmax;
-                            g.dens_f = 1.f;
-                            g.dL0 = st.dL0;
-                            g.dR0 = st.dR0;
-                            g.two_zr = st.two_zr;
-                            g.inv_h2 = st.inv_h2;
-                            g.ch = st.ch;
-                            // unit density: the single-channel form multiplies this by dens
-                            f32 = colden_interior32(g, a.lp.kernel, (float)btk, k);
-                        }
-#pragma unroll
-                        for (int c = 0; c < MAX_CHANNELS; c++)
-                            if (live[c]) {
-                                const float v = edge ? (float)((double)st.dens[c] * fe)
-                                                     : st.dens[c] * f32;
-                                accumulate<float, 1>(a.dev_err, v, j, S[c],
-                                                     acc + 2 * (size_t)c * nbins,
-                                                     acc + (2 * (size_t)c + 1) * nbins,
-                                                     &s_bad[c]);
-                            }
+                    const bool edge = k == 0 || k >= st.kmax - 1;
+                    const double fe = k == 0 ? st.kf0 : (k == st.kmax ? st.kf2 : st.kf1);
+                    float f32 = 0.f;
+                    if (!edge) {
+                        StageCol32 g;
+                        g.kmax = st.kmax;
+                        g.dens_f = 1.f;
+                        g.dL0 = st.dL0;
+                        g.dR0 = st.dR0;
+                        g.two_zr = st.two_zr;
+                        g.inv_h2 = st.inv_h2;
+                        g.ch = st.ch;
+                        // unit density: the single-channel form multiplies this by dens
+                        f32 = colden_interior32(g, a.lp.kernel, (float)btk, k);
                     }
+#pragma unroll
+                    for (int c = 0; c < MAX_CHANNELS; c++)
+                        if (live[c]) {
+                            const float v = edge ? (float)((double)st.dens[c] * fe)
+                                                 : st.dens[c] * f32;
+                            accumulate<float, 1>(a.dev_err, v, j, S[c],
+                                                 acc + 2 * (size_t)c * nbins,
+                                                 acc + (2 * (size_t)c + 1) * nbins,
+                                                 &s_bad[c]);
+                        }
                     j += 32;
                     while (j >= nbins)
                         j -= nbins;
@@ -2670,7 +2681,7 @@ size_t deposit_smem_bytes(const DepositLaunch &cfg, int compute_tau, int nbins)
         return (cfg.smem_mode ? (size_t)16 * nbins : 0) +
                (size_t)16 * tiles64_layout(cfg.tiles, nbins).nodes +
                (size_t)(cfg.threads / 32) * cfg.chunk *
-                   sizeof(Stage64) +
+                   (compute_tau ? sizeof(Stage64) : sizeof(StageC64)) +
                (cfg.table ? sizeof(FixRow) * FSG_FIX_ROWS : 0);
     return (cfg.smem_mode ? (size_t)16 * nbins : 0) +
            (size_t)(cfg.threads / 32) * cfg.chunk * stage_pair_bytes(compute_tau, cfg.precision) +
@@ -2702,6 +2713,18 @@ void plan_tau64(DepositLaunch &cfg, int nbins, size_t cap)
     cfg.table = 1;
     cfg.table = deposit_smem_bytes(cfg, 1, nbins) <= cap;
     for (cfg.chunk = T64_CHUNK; cfg.chunk > 1 && deposit_smem_bytes(cfg, 1, nbins) > cap;)
+        cfg.chunk /= 2;
+}
+
+// FP64 column densities: 32 staged pairs per warp (full warps for the FP64
+// pixels), fewer where the accumulators leave less room.
+void plan_colden64(DepositLaunch &cfg, int nbins, size_t cap)
+{
+    const size_t stage_min = (size_t)(C64_THREADS / 32) * (C64_CHUNK / 4) * sizeof(StageC64);
+    cfg.smem_mode = (size_t)16 * nbins + stage_min <= cap;
+    cfg.tiles = 0;
+    cfg.table = 0;
+    for (cfg.chunk = C64_CHUNK; cfg.chunk > 1 && deposit_smem_bytes(cfg, 0, nbins) > cap;)
         cfg.chunk /= 2;
 }
 }  // namespace
@@ -2743,7 +2766,10 @@ void deposit_plan(DepositLaunch &cfg, int compute_tau, int nbins)
     }
     cfg.chunk = 0;
     if (cfg.fast64) {
-        plan_tau64(cfg, nbins, cap);
+        if (compute_tau)
+            plan_tau64(cfg, nbins, cap);
+        else
+            plan_colden64(cfg, nbins, cap);
         return;
     }
     cfg.tiles = 0;
@@ -2759,8 +2785,7 @@ int deposit_max_smem_bins(int compute_tau, int precision, int threads)
 namespace {
 decltype(&fast64_kernel<true>) fast64_build(int compute_tau)
 {
-    (void)compute_tau;
-    return fast64_kernel<true>;
+    return compute_tau ? fast64_kernel<true> : fast64_kernel<false>;
 }
 
 cudaLaunchConfig_t fast64_launch(int compute_tau, int grid, int threads, size_t smem, int cluster,
@@ -2969,7 +2994,8 @@ int chan_threads(int precision) { return precision == 0 ? 256 : 512; }
 size_t chan_smem(int precision, int nch, int nbins, int smem_mode)
 {
     return (smem_mode ? 2 * sizeof(unsigned long long) * nbins * nch : 0) +
-           (size_t)(chan_threads(precision) / 32) * CHAN_CHUNK * sizeof(StageColK);
+           (size_t)(chan_threads(precision) / 32) * CHAN_CHUNK *
+               (sizeof(StageColK) + (precision == 0 ? sizeof(StageC64) : 0));
 }
 template <int PREC>
 void chan_attr(size_t smem)

@@ -88,10 +88,9 @@ __device__ __forceinline__ void nodes_to_coefs64(double *node, int ntiles)
 }
 
 template <bool TAU>
-__global__ void __launch_bounds__(T64_THREADS, 1) fast64_kernel(DepositArgs a)
+__global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_kernel(DepositArgs a)
 {
-    static_assert(TAU, "optical depth");
-    using Stage = Stage64;
+    using Stage = typename std::conditional<TAU, Stage64, StageC64>::type;
     extern __shared__ __align__(16) unsigned long long smem[];
     __shared__ BoundScratch red;
     __shared__ int s_bad;
@@ -177,8 +176,11 @@ __global__ void __launch_bounds__(T64_THREADS, 1) fast64_kernel(DepositArgs a)
                 if (cb >= e1)
                     break;
                 const int n = (int)min((long long)a.chunk, e1 - cb);
-                deposit_tau64(a, tl, rows, axis, cb, n, S, lo, hi, tlo, thi, &s_bad, stage, bintov,
-                              lane);
+                if constexpr (TAU)
+                    deposit_tau64(a, tl, rows, axis, cb, n, S, lo, hi, tlo, thi, &s_bad, stage,
+                                  bintov, lane);
+                else
+                    deposit_colden64(a, axis, cb, n, S, lo, hi, &s_bad, stage, btk, lane);
             }
         }
         cluster_sync();

@@ -303,7 +303,7 @@ int noalloc_run(int compute_tau, int nbins, int kernel, double box, double velfa
         cfg.precision = precision;
         cfg.threads = threads;
         cfg.tiles = 1;
-        cfg.fast64 = precision == FSG_PREC_FP64 && compute_tau;
+        cfg.fast64 = precision == FSG_PREC_FP64;
         if (cfg.fast64) {
             cfg.threads = 512;
             deposit_plan(cfg, compute_tau, nbins);
