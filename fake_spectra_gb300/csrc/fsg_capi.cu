@@ -1146,43 +1146,6 @@ fsg_context *default_context()
     return g_default[dev];
 }
 
-// Pairs of every sightline in ascending particle order (the reference's
-// std::map order, which the Voronoi cell assignment depends on).
-void sort_pairs_by_particle(fsg_context *c)
-{
-    const long long total = c->npairs;
-    if (total <= 0)
-        return;
-    cudaStream_t s = c->stream;
-    std::vector<int> part((size_t)total);
-    std::vector<double> dr2((size_t)total);
-    cuda_check(cudaMemcpyAsync(part.data(), c->part.p, sizeof(int) * total, cudaMemcpyDeviceToHost,
-                               s), "D2H pairs");
-    cuda_check(cudaMemcpyAsync(dr2.data(), c->dr2.p, sizeof(double) * total,
-                               cudaMemcpyDeviceToHost, s), "D2H pairs");
-    cuda_check(cudaStreamSynchronize(s), "D2H pairs");
-    std::vector<std::pair<int, double>> tmp;
-    for (int l = 0; l < c->nlos; l++) {
-        const long long a = c->h_off[l], b = c->h_off[l + 1];
-        tmp.resize((size_t)(b - a));
-        for (long long e = a; e < b; e++)
-            tmp[e - a] = {part[e], dr2[e]};
-        std::sort(tmp.begin(), tmp.end(),
-                  [](const std::pair<int, double> &x, const std::pair<int, double> &y) {
-                      return x.first < y.first;
-                  });
-        for (long long e = a; e < b; e++) {
-            part[e] = tmp[e - a].first;
-            dr2[e] = tmp[e - a].second;
-        }
-    }
-    cuda_check(cudaMemcpyAsync(c->part.p, part.data(), sizeof(int) * total, cudaMemcpyHostToDevice,
-                               s), "H2D pairs");
-    cuda_check(cudaMemcpyAsync(c->dr2.p, dr2.data(), sizeof(double) * total,
-                               cudaMemcpyHostToDevice, s), "H2D pairs");
-    cuda_check(cudaStreamSynchronize(s), "H2D pairs");
-}
-
 // IndexTable::assign_cells for every sightline: the segment of each pair's cell.
 const float2 *voronoi_cells(fsg_context *c, const Particles &p, const double *cofm, double box)
 {
@@ -1194,7 +1157,6 @@ const float2 *voronoi_cells(fsg_context *c, const Particles &p, const double *co
         fail(FSG_ERR_VALUE, "box %g too large for the Voronoi sightline grid (0.1 kpc/h points)",
              box);
     cudaStream_t s = c->stream;
-    sort_pairs_by_particle(c);
     auto *seg = (float2 *)c->ensure(c->vseg, sizeof(float2) * total);
     auto *scratch = (int *)c->ensure(c->vscratch,
                                      sizeof(int) * voronoi_scratch_ints(total, nlos));
@@ -1205,7 +1167,7 @@ const float2 *voronoi_cells(fsg_context *c, const Particles &p, const double *co
     cuda_check(cudaMemsetAsync(err, 0, sizeof(unsigned), s), "memset");
     launch_voronoi_cells(p.pos, (const int *)c->part.p, (const long long *)c->off.p,
                          c->tables.axis, dcofm, nlos, total, box, scratch, seg, err, s);
-    c->stats.gpu_launches += 10;
+    c->stats.gpu_launches += 1 + 4 * ((nlos + 65534) / 65535);
     cuda_check(cudaGetLastError(), "Voronoi cells launch");
     unsigned h_err = 0;
     cuda_check(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read");

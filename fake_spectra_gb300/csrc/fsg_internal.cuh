@@ -200,8 +200,8 @@ void launch_colden_channels(const LineParams &lp, const LineTables &t, const Par
                             int grid, cudaStream_t s);
 
 // Voronoi-mesh cells (fsg_voronoi.cu): seg[P] = the [left, right] segment
-// of each pair's cell along its sightline (IndexTable::assign_cells); the
-// pairs of a sightline must be in ascending particle order.  scratch holds
+// of each pair's cell along its sightline (IndexTable::assign_cells), for pair
+// lists in any order (ties go to the smaller particle index).  scratch holds
 // voronoi_scratch_ints(P, L) ints; cofm is a device copy (3L doubles).
 long long voronoi_scratch_ints(long long npairs, int nlos);
 void launch_voronoi_cells(const float *pos, const int *part, const long long *off,
