@@ -99,6 +99,7 @@ struct fsg_context {
     DevBuf vseg, vscratch, vcofm;                            // Voronoi cells
     DevBuf tune_order;                                       // autotuner sample
     DevBuf prec;                                             // pair records (FP32 tau)
+    DevBuf split;                                            // shared sightlines (FP64)
     HostBuf hstage;   // host-pointer entries: pinned staging of inputs and output
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t cp[2] = {nullptr, nullptr};   // copy timing of the host-pointer entries
@@ -181,7 +182,7 @@ struct fsg_context {
                           &skey, &sperm, &shist, &sstart, &ssums, &flag, &tcount, &tstart,
                           &tsums, &idx, &fpart, &fout, &fedges, &fcounts, &ftau, &fdflux,
                           &ffft, &fpower, &ptables, &pchirp, &pbhat, &ppart, &fexp, &vseg,
-                          &vscratch, &vcofm, &tune_order, &prec, &gorder};
+                          &vscratch, &vcofm, &tune_order, &prec, &split, &gorder};
         pplan = PowerPlan{};
         fexp_ready = false;
         for (DevBuf *b : bufs) {
@@ -547,7 +548,9 @@ void deposit(fsg_context *c, const LineParams &lp, const Particles &p, double *o
         ctr = (unsigned long long *)c->ensure(c->counters, sizeof(unsigned long long) * 8);
         cuda_check(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * 8, s), "memset");
     }
-    const int G = (rows && rows->groups > 1 && !count && nlos >= 64 * rows->groups)
+    // sightlines few enough to be shared between blocks are launched at once
+    const int G = (rows && rows->groups > 1 && !count && !cfg.split_ws &&
+                   nlos >= 64 * rows->groups)
                       ? std::min(rows->groups, (int)fsg_context::ROW_GROUPS)
                       : 1;
     auto *ticket = (unsigned *)c->ensure(c->ticket, sizeof(unsigned) * G);
@@ -670,7 +673,8 @@ DepositLaunch deposit_config(fsg_context *c, const LineParams &lp, const fsg_opt
     if (opt && opt->records > 1)
         fail(FSG_ERR_VALUE, "records must be -1 (tuned), 0 or 1");
     cfg.fast64 = cfg.precision == FSG_PREC_FP64 && !count;
-    const int tdef = cfg.precision == FSG_PREC_FP64 && !cfg.fast64 ? 256 : 512;
+    const int tdef = cfg.fast64 ? fast64_threads(lp.compute_tau)
+                                : (cfg.precision == FSG_PREC_FP64 ? 256 : 512);
     const int tmax = cfg.precision == FSG_PREC_FP64 ? 256 : (tau32 ? 1024 : 512);
     cfg.threads = (opt && opt->threads > 0 && !vor) ? opt->threads : tdef;
     if (opt && opt->threads > 0 && !vor && (cfg.threads % 32 || cfg.threads > tmax))
@@ -798,13 +802,12 @@ fsg_tune_key tune_key(fsg_context *c, const LineParams &lp, int precision)
 void finish_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
 {
     int sms = 0;
-    if (cfg.fast64) {
-        deposit_clusters(cfg, lp.compute_tau, lp.nbins, c->nlos);
-        return;
-    }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     const int per_sm = std::max(1, deposit_resident_ctas(cfg, lp.compute_tau, lp.nbins));
-    cfg.grid = std::min(c->nlos, sms * per_sm);
+    deposit_fit_chunk(cfg, c->npairs, sms);
+    const size_t sb = deposit_split_bytes(cfg, lp.nbins, c->nlos, sms);
+    cfg.split_ws = sb ? c->ensure(c->split, sb) : nullptr;
+    cfg.grid = sb ? sms * per_sm : std::min(c->nlos, sms * per_sm);
 }
 
 // Times the candidate launches on a sample of the call's sightlines (every
@@ -1019,7 +1022,7 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
         put(cfgs[k].chunk);
         put(cfgs[k].tiles);
         put(cfgs[k].rec);
-        put(cfgs[k].cluster);
+        putp(cfgs[k].split_ws);
     }
     cudaStream_t s = c->own;
     cuda_check(cudaStreamSynchronize(c->stream), "sync caller stream");

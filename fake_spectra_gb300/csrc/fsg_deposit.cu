@@ -1339,6 +1339,7 @@ struct DepositArgs {
     int tiles;                      // far-field tile accumulators (FP64 tau: the width of
                                     // the narrowest tiles)
     int table_off;                  // FP64 tau: byte offset of the staged K table, 0 = none
+    void *split_ws;                 // fast64_kernel: state of shared sightlines, or null
 };
 
 // FMT 0: 128-bit fixed point with carries (FP64 form); 1: split (FP32 form).
@@ -2690,13 +2691,13 @@ size_t deposit_smem_bytes(const DepositLaunch &cfg, int compute_tau, int nbins)
 
 namespace {
 // FP64 optical depths through fast64_kernel.  The tile layout depends on nbins
-// only (room is kept for 16 warps of 4 staged pairs), so that every launch
+// only (room is kept for 64 staged pairs), so that every launch
 // sums the same values: the narrowest first tiles that fit, 64 pixels (up to
 // 8600 bins on GB300) to 256; accumulators go to global memory when they do
 // not fit beside the staged pairs.
 void plan_tau64(DepositLaunch &cfg, int nbins, size_t cap)
 {
-    const size_t stage_min = (size_t)(T64_THREADS / 32) * (T64_CHUNK / 2) * sizeof(Stage64);
+    const size_t stage_min = (size_t)64 * sizeof(Stage64);
     const size_t acc = (size_t)16 * nbins;
     const int asked = cfg.tiles;
     cfg.fast64 = 1;
@@ -2709,7 +2710,7 @@ void plan_tau64(DepositLaunch &cfg, int nbins, size_t cap)
                 cfg.tiles = w0;
     // the K table (30 KB) in shared memory where 4 staged pairs still fit, else
     // it is read through L1
-    cfg.chunk = T64_CHUNK / 2;
+    cfg.chunk = 64 / (T64_THREADS / 32);
     cfg.table = 1;
     cfg.table = deposit_smem_bytes(cfg, 1, nbins) <= cap;
     for (cfg.chunk = T64_CHUNK; cfg.chunk > 1 && deposit_smem_bytes(cfg, 1, nbins) > cap;)
@@ -2788,60 +2789,41 @@ decltype(&fast64_kernel<true>) fast64_build(int compute_tau)
     return compute_tau ? fast64_kernel<true> : fast64_kernel<false>;
 }
 
-cudaLaunchConfig_t fast64_launch(int compute_tau, int grid, int threads, size_t smem, int cluster,
-                                 cudaLaunchAttribute *attr, cudaStream_t s)
+int fast64_resident(int compute_tau, int threads, size_t smem)
 {
-    cudaFuncSetAttribute(fast64_build(compute_tau), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3((unsigned)grid);
-    lc.blockDim = dim3((unsigned)threads);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = s;
-    attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = (unsigned)cluster;
-    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    return lc;
-}
-
-// Clusters of `cluster` fast64_kernel blocks that the device holds at once.
-int fast64_clusters(int compute_tau, int threads, size_t smem, int cluster)
-{
-    cudaLaunchAttribute attr{};
-    const cudaLaunchConfig_t lc = fast64_launch(compute_tau, cluster, threads, smem, cluster,
-                                                &attr, 0);
+    auto k = fast64_build(compute_tau);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, fast64_build(compute_tau), &lc) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 0;
-    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem);
     return n;
 }
 }  // namespace
 
-// The cluster size with the least time for `nlos` equal sightlines, counting
-// whole waves: a wave of n clusters of c blocks takes 1/c of a sightline's
-// time, and each doubling costs a few percent (barriers, the shared sum).
-void deposit_clusters(DepositLaunch &cfg, int compute_tau, int nbins, int nlos)
+int fast64_threads(int compute_tau) { return compute_tau ? T64_THREADS : C64_THREADS; }
+
+// Smaller chunks for small calls: at least four per warp of the whole device
+// (down to 2 pairs; the set-up of a chunk fills fewer lanes, but 22 thousand
+// pairs in chunks of 8 leave a third of the warps without one).
+void deposit_fit_chunk(DepositLaunch &cfg, long long npairs, int sms)
 {
-    const size_t smem = deposit_smem_bytes(cfg, compute_tau, nbins);
-    double best = 1e300;
-    cfg.cluster = 1;
-    cfg.grid = nlos;
-    double penalty = 1.0;
-    for (int c = 1; c <= (cfg.smem_mode ? 8 : 1); c *= 2, penalty *= 1.04) {
-        const int n = fast64_clusters(compute_tau, cfg.threads, smem, c);
-        if (n <= 0)
-            continue;
-        const double t = penalty * std::ceil((double)nlos / n) / c;
-        if (t < best) {
-            best = t;
-            cfg.cluster = c;
-            cfg.grid = c * std::min(nlos, n);
-        }
-    }
+    if (!cfg.fast64)
+        return;
+    while (cfg.chunk > 2 && npairs < 4ll * sms * (cfg.threads / 32) * cfg.chunk)
+        cfg.chunk /= 2;
+}
+
+// Blocks help each other's sightlines (fast64_kernel) while a block has few of
+// them, 8 on average: beyond that the queue's tail is short against the whole,
+// and the words in global memory would grow (16 bytes a pixel and tile node of
+// every sightline; at most SPLIT_MAX bytes).  Also for nonpersistent launches:
+// never.
+size_t deposit_split_bytes(const DepositLaunch &cfg, int nbins, int nlos, int sms)
+{
+    constexpr size_t SPLIT_MAX = (size_t)1 << 29;
+    if (!cfg.fast64 || !cfg.smem_mode || !cfg.persistent || nlos > 8 * sms)
+        return 0;
+    const size_t b = split_bytes(nlos, nbins, tiles64_layout(cfg.tiles, nbins).nodes);
+    return b <= SPLIT_MAX ? b : 0;
 }
 
 int deposit_resident_ctas(const DepositLaunch &cfg, int compute_tau, int nbins)
@@ -2849,7 +2831,7 @@ int deposit_resident_ctas(const DepositLaunch &cfg, int compute_tau, int nbins)
     const size_t smem = deposit_smem_bytes(cfg, compute_tau, nbins);
     const int threads = cfg.threads;
     if (cfg.fast64)
-        return fast64_clusters(compute_tau, threads, smem, 1);
+        return fast64_resident(compute_tau, threads, smem);
     if (compute_tau)
         return cfg.precision ? resident_ctas<true, 1, false>(threads, smem, cfg.rec != 0)
                              : resident_ctas<true, 0, false>(threads, smem, false);
@@ -2889,14 +2871,15 @@ int launch_deposit(const LineParams &lp, const LineTables &t, const Particles &p
     const size_t smem = deposit_smem_bytes(cfg, lp.compute_tau, lp.nbins);
     int launched = 1;
     if (cfg.fast64 && counters == nullptr) {
-        const int c = std::max(1, cfg.cluster);
         a.table_off = cfg.table ? (int)(smem - sizeof(FixRow) * FSG_FIX_ROWS) : 0;
-        cudaLaunchAttribute attr{};
-        const cudaLaunchConfig_t lc = fast64_launch(
-            lp.compute_tau,
-            cfg.persistent ? std::max(c, std::min(cfg.grid, c * nlos)) : c * nlos, cfg.threads,
-            smem, c, &attr, s);
-        cudaLaunchKernelEx(&lc, fast64_build(lp.compute_tau), a);
+        a.split_ws = cfg.split_ws;
+        auto k = fast64_build(lp.compute_tau);
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (a.split_ws)
+            cudaMemsetAsync(a.split_ws, 0,
+                            split_bytes(nlos, lp.nbins,
+                                        tiles64_layout(cfg.tiles, lp.nbins).nodes), s);
+        k<<<cfg.persistent ? cfg.grid : nlos, cfg.threads, smem, s>>>(a);
         return launched;
     }
     if (cfg.tiles && counters == nullptr) {

@@ -1,52 +1,94 @@
 // Kernel skeleton of the FP64 deposits (included by fsg_deposit.cu inside its
 // anonymous namespace): sightlines from a queue, 128-bit accumulators in
 // shared memory (or global memory for very long rows), chunks of pairs dealt to
-// the warps, and optionally a thread-block cluster per sightline, whose blocks
-// sum their accumulators through distributed shared memory.
+// the warps.
+//
+// Pair costs differ by orders of magnitude and sightlines are often few, so a
+// block that finds the queue empty helps: it takes chunks from the sightline
+// with the most left, adds them in its own accumulators and then adds those
+// into the sightline's words in global memory.  The block whose chunks complete
+// the sightline writes the row.  Sums are integers, so the bits do not depend
+// on who did what.  (Without help 72 sightlines through a clumpy 128^3 snapshot
+// left the SMs idle for 69% of the kernel, and 37% with a cluster of four
+// blocks per sightline.)
 
-__device__ __forceinline__ unsigned cluster_size()
+// Per-launch state of shared sightlines, zeroed before the launch.
+struct SplitState {
+    unsigned *next, *done;   // [nlos] chunks taken, chunks whose sums are in acc
+    unsigned *ready;         // [nlos] B is set and chunks may be taken
+    unsigned *active;        // [nlos] blocks that have joined (a hint)
+    unsigned *bad;           // [nlos] a contribution was not finite
+    unsigned *started;       // sightlines that are ready or need no chunks
+    double *B;               // [nlos] bound of the sightline total
+    unsigned long long *acc;     // [nlos][2 (nbins + nodes)]
+    size_t words;            // 2 (nbins + nodes)
+};
+
+size_t split_bytes(int nlos, int nbins, int nodes)
 {
-    unsigned n;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
-    return n;
-}
-__device__ __forceinline__ unsigned cluster_rank()
-{
-    unsigned r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// Barrier of every thread of the cluster (release / acquire).
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The address of this block's shared object in the block of rank r.
-template <class T>
-__device__ __forceinline__ T *cluster_map(T *p, unsigned r)
-{
-    unsigned long long out;
-    asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"((unsigned long long)p), "r"(r));
-    return reinterpret_cast<T *>(out);
+    return 64 + (size_t)nlos * (5 * sizeof(unsigned) + sizeof(double) + 4 +
+                                sizeof(unsigned long long) * 2 * ((size_t)nbins + nodes));
 }
 
-// Sum over the cluster's blocks of a 128-bit accumulator word, as a double.
-__device__ __forceinline__ double cluster_fixed(unsigned long long *lo, unsigned long long *hi,
-                                                unsigned nc, int S)
+__host__ __device__ inline SplitState split_state(void *ws, int nlos, int nbins, int nodes)
 {
-    unsigned long long l = lo[0], h = hi[0];
-    if (nc > 1) {
-        l = 0ull;
-        h = 0ull;
-        for (unsigned r = 0; r < nc; r++) {
-            const unsigned long long x = *cluster_map(lo, r);
-            h += *cluster_map(hi, r);
-            l += x;
-            h += l < x ? 1ull : 0ull;
+    SplitState st;
+    st.words = 2 * ((size_t)nbins + nodes);
+    unsigned char *p = (unsigned char *)ws;
+    st.acc = (unsigned long long *)p;
+    p += sizeof(unsigned long long) * st.words * nlos;
+    st.B = (double *)p;
+    p += sizeof(double) * nlos;
+    unsigned *u = (unsigned *)p;
+    st.next = u;
+    st.done = u + nlos;
+    st.ready = u + 2 * (size_t)nlos;
+    st.active = u + 3 * (size_t)nlos;
+    st.bad = u + 4 * (size_t)nlos;
+    st.started = u + 5 * (size_t)nlos;
+    return st;
+}
+
+__device__ __forceinline__ unsigned ld_cg(const unsigned *p) { return __ldcg(p); }
+
+// The sightline with the most chunks left per block working on it, or -1 (whole
+// block).  Waits a while for sightlines whose bound is still being formed: at
+// most SPLIT_POLLS polls, after which the block leaves (the owners need no help).
+constexpr int SPLIT_POLLS = 4096;
+__device__ int pick_line(const DepositArgs &a, const SplitState &sp, unsigned min_left,
+                         unsigned long long *s_best)
+{
+    for (int poll = 0; poll < SPLIT_POLLS; poll++) {
+        const bool all = ld_cg(sp.started) >= (unsigned)a.nlos;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            *s_best = 0ull;
+        __syncthreads();
+        for (int i = threadIdx.x; i < a.nlos; i += blockDim.x) {
+            const int l = a.line_order[i];
+            if (!ld_cg(&sp.ready[i]))
+                continue;
+            const long long n = (a.pl.off[l + 1] - a.pl.off[l] + a.chunk - 1) / a.chunk;
+            const long long left = n - (long long)ld_cg(&sp.next[i]);
+            if (left < (long long)min_left)
+                continue;
+            const unsigned score = (unsigned)min(left * 16 / (1 + (long long)ld_cg(&sp.active[i])),
+                                                 0x7fffffffll);
+            atomicMax(s_best, ((unsigned long long)score << 32) | (unsigned)(i + 1));
         }
+        __syncthreads();
+        const unsigned long long b = *s_best;
+        if (b) {
+            const int i = (int)(unsigned)b - 1;
+            if (threadIdx.x == 0)
+                atomicAdd(&sp.active[i], 1u);
+            return i;
+        }
+        if (__syncthreads_and(all))
+            return -1;
+        __nanosleep(500);
     }
-    return from_fixed(l, h, S);
+    return -1;
 }
 
 // Clenshaw sum of the M Chebyshev coefficients c at t in [-1, 1].
@@ -93,14 +135,16 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
     using Stage = typename std::conditional<TAU, Stage64, StageC64>::type;
     extern __shared__ __align__(16) unsigned long long smem[];
     __shared__ BoundScratch red;
+    __shared__ unsigned long long s_best;
     __shared__ int s_bad;
-    __shared__ unsigned s_ticket, s_chunk;
+    __shared__ unsigned s_ticket, s_chunk, s_mine, s_last;
     const int nbins = a.lp.nbins;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned nc = cluster_size(), rank = cluster_rank();
     const double bintov = a.lp.vbox / nbins;
     const double btk = a.lp.vbox / nbins / a.lp.velfac;
     const Tiles64 tl = tiles64_layout(a.tiles, nbins);
+    const bool split = a.split_ws != nullptr;
+    const SplitState sp = split_state(a.split_ws, a.nlos, nbins, tl.nodes);
     // dynamic shared memory: [accumulators lo, hi (smem_mode)] [tile nodes lo, hi] [stage]
     // [K table]
     unsigned long long *tlo = smem + (a.smem_mode ? 2 * (size_t)nbins : 0);
@@ -109,6 +153,8 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
                                              2 * (size_t)tl.nodes) + warp * a.chunk;
     for (int j = threadIdx.x; TAU && j < 64; j += blockDim.x) {
         s_cos64[j] = cospi((double)j / 32.0);
+        if (j < T64_M)
+            s_node64[j] = 0.5 + 0.5 * cospi((double)(2 * j + 1) / 32.0);
         s_pow2[j] = d_fix_pow2[j];
     }
     Rows64 rows{d_fix_rows, 0};
@@ -119,29 +165,36 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
             dst[j ^ ((j >> 3) & 3)] = src[j];
         rows = Rows64{reinterpret_cast<const FixRow *>(dst), 3};
     }
-    const unsigned first = blockIdx.x / nc;
-    unsigned ticket = first;
-    for (;;) {
-        if (a.persistent) {
-            // the cluster's first block draws the next sightline
-            if (rank == 0 && threadIdx.x == 0) {
-                const unsigned t = atomicAdd(a.ticket, 1u);
-                for (unsigned r = 0; r < nc; r++)
-                    *cluster_map(&s_ticket, r) = t;
-            }
-            cluster_sync();
-            ticket = s_ticket;
+    for (bool first = true;; first = false) {
+        // the next sightline (its place in the queue): an own one, else one to help with
+        __syncthreads();
+        if (threadIdx.x == 0)
+            s_ticket = a.persistent ? atomicAdd(a.ticket, 1u) : (first ? blockIdx.x : 0xFFFFFFFFu);
+        __syncthreads();
+        int q = (int)min(s_ticket, 0x7fffffffu);
+        const bool owner = q < a.nlos;
+        if (!owner) {
+            if (!split)
+                break;
+            q = pick_line(a, sp, (unsigned)(blockDim.x >> 5), &s_best);
+            if (q < 0)
+                break;
         }
-        if (ticket >= (unsigned)a.nlos)
-            break;
-        const int line = a.line_order[ticket];
+        const int line = a.line_order[q];
         const int axis = a.t.axis[line];
         const long long e0 = a.pl.off[line], e1 = a.pl.off[line + 1];
-        const auto bound = [&](long long e) {
-            const PairInput in = load_pair(a.p, a.pl, e, axis, TAU, a.dev_err);
-            return TAU ? tau_pair_bound(a.lp, in) : colden_pair_bound(a.lp, in, btk);
-        };
-        const double B = order_free_bound(e0, e1, bound, bound, &red);
+        const unsigned nchunks = (unsigned)((e1 - e0 + a.chunk - 1) / a.chunk);
+        double B;
+        if (owner) {
+            const auto bound = [&](long long e) {
+                const PairInput in = load_pair(a.p, a.pl, e, axis, TAU, a.dev_err);
+                return TAU ? tau_pair_bound(a.lp, in) : colden_pair_bound(a.lp, in, btk);
+            };
+            B = order_free_bound(e0, e1, bound, bound, &red);
+        } else {
+            B = __ldcg(&sp.B[q]);
+        }
+        const bool live = isfinite(B) && B > 0.0;
         unsigned long long *lo, *hi;
         if (a.smem_mode) {
             lo = smem;
@@ -160,21 +213,30 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
         }
         if (threadIdx.x == 0) {
             s_chunk = 0u;
+            s_mine = 0u;
             s_bad = !isfinite(B);
+            if (owner && split) {
+                sp.B[q] = B;
+                __threadfence();
+                if (live)
+                    atomicExch(&sp.ready[q], 1u);
+                atomicAdd(sp.started, 1u);
+            }
         }
-        cluster_sync();
-        const bool live = isfinite(B) && B > 0.0;
+        __syncthreads();
         const int S = live ? 124 - ilogb(B) : 0;
         if (live) {
-            unsigned *counter = cluster_map(&s_chunk, 0);
+            unsigned *counter = split ? &sp.next[q] : &s_chunk;
+            unsigned mine = 0;
             for (;;) {
                 unsigned c = 0;
                 if (lane == 0)
                     c = atomicAdd(counter, 1u);
                 c = __shfl_sync(0xffffffffu, c, 0);
-                const long long cb = e0 + (long long)c * a.chunk;
-                if (cb >= e1)
+                if (c >= nchunks)
                     break;
+                mine++;
+                const long long cb = e0 + (long long)c * a.chunk;
                 const int n = (int)min((long long)a.chunk, e1 - cb);
                 if constexpr (TAU)
                     deposit_tau64(a, tl, rows, axis, cb, n, S, lo, hi, tlo, thi, &s_bad, stage,
@@ -182,29 +244,56 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
                 else
                     deposit_colden64(a, axis, cb, n, S, lo, hi, &s_bad, stage, btk, lane);
             }
+            if (lane == 0 && mine)
+                atomicAdd(&s_mine, mine);
         }
-        cluster_sync();
+        __syncthreads();
         bool bad = s_bad != 0;
-        for (unsigned r = 0; r < nc && !bad; r++)
-            bad = *cluster_map(&s_bad, r) != 0;
+        if (live && split && s_mine != nchunks) {
+            // a shared sightline: this block's sums go to its words in global
+            // memory, and the block that completes it takes them back
+            const unsigned mine = s_mine;
+            if (mine == 0u)
+                continue;
+            unsigned long long *g = sp.acc + (size_t)q * sp.words;
+            const auto merge = [&](unsigned long long *l, unsigned long long *h, size_t at, int n) {
+                for (int j = threadIdx.x; j < n; j += blockDim.x)
+                    if (l[j] | h[j])
+                        fixed_add(g + at, g + at + n, j, l[j], h[j]);
+            };
+            merge(lo, hi, 0, nbins);
+            merge(tlo, thi, 2 * (size_t)nbins, tl.nodes);
+            if (threadIdx.x == 0 && bad)
+                atomicOr(&sp.bad[q], 1u);
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0)
+                s_last = atomicAdd(&sp.done[q], mine) + mine == nchunks;
+            __syncthreads();
+            if (!s_last)
+                continue;
+            __threadfence();
+            for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
+                lo[j] = __ldcg(g + j);
+                hi[j] = __ldcg(g + nbins + j);
+            }
+            for (int j = threadIdx.x; j < tl.nodes; j += blockDim.x) {
+                tlo[j] = __ldcg(g + 2 * (size_t)nbins + j);
+                thi[j] = __ldcg(g + 2 * (size_t)nbins + tl.nodes + j);
+            }
+            bad = ld_cg(&sp.bad[q]) != 0u;
+            __syncthreads();
+        }
         if (bad) {
-            if (rank == 0 && threadIdx.x == 0)
+            if (threadIdx.x == 0)
                 a.bad_lines[atomicAdd(a.n_bad, 1)] = line;
         } else if (live) {
             double *row = a.out + (size_t)line * nbins;
             double *node = reinterpret_cast<double *>(tlo);
             if (tl.nodes > 0) {
-                // node sums as doubles: each block forms its share for all blocks
-                for (int j = rank * blockDim.x + threadIdx.x; j < tl.nodes;
-                     j += nc * blockDim.x) {
-                    const double v = cluster_fixed(tlo + j, thi + j, nc, S);
-                    if (nc == 1)
-                        node[j] = v;
-                    else
-                        for (unsigned r = 0; r < nc; r++)
-                            *cluster_map(node + j, r) = v;
-                }
-                cluster_sync();
+                for (int j = threadIdx.x; j < tl.nodes; j += blockDim.x)
+                    node[j] = from_fixed(tlo[j], thi[j], S);
+                __syncthreads();
                 // from the widest tiles down: coefficients, added at the nodes
                 // of the four tiles below
                 for (int l = T64_LEVELS - 1; l >= 0; l--) {
@@ -226,16 +315,14 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
             }
             const int covered = tl.w0 > 0 ? nbins / tl.w0 * tl.w0 : 0;
             const double inv_w = tl.w0 > 0 ? 2.0 / tl.w0 : 0.0;
-            for (int j = rank * blockDim.x + threadIdx.x; j < nbins; j += nc * blockDim.x) {
-                double v = cluster_fixed(lo + j, hi + j, nc, S);
+            for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
+                double v = from_fixed(lo[j], hi[j], S);
                 if (j < covered)
                     v += clenshaw64(node + (size_t)(j / tl.w0) * T64_M,
                                     fma((double)(j & (tl.w0 - 1)) + 0.5, inv_w, -1.0));
                 row[j] = v;
             }
         }
-        // no block clears or leaves its accumulators while another reads them
-        cluster_sync();
         if (!a.persistent)
             break;
     }

@@ -288,7 +288,7 @@ struct DepositLaunch {
     int rec;                 // FP32 tau: through pair records (PairLists::rec must be set)
     int fast64;              // FP64 through fast64_kernel (planned with smem_mode)
     int table;               // fast64_kernel, tau: K table staged in shared memory
-    int cluster;             // fast64_kernel: blocks that share a sightline
+    void *split_ws;          // fast64_kernel: deposit_split_bytes() of device memory, or null
 };
 
 // Deposits all pairs of all sightlines into out[L*nbins] (pre-zeroed).  Lines
@@ -307,8 +307,12 @@ int launch_deposit(const LineParams &lp, const LineTables &t, const Particles &p
 void deposit_plan(DepositLaunch &cfg, int compute_tau, int nbins);
 // Dynamic shared memory of one deposit CTA.
 size_t deposit_smem_bytes(const DepositLaunch &cfg, int compute_tau, int nbins);
-// fast64_kernel (cfg.fast64): blocks per cluster and the grid for nlos sightlines.
-void deposit_clusters(DepositLaunch &cfg, int compute_tau, int nbins, int nlos);
+// fast64_kernel (cfg.fast64): device memory that lets blocks help each other with
+// a sightline (cleared by launch_deposit), 0 = not worth it; deposit_fit_chunk
+// makes the planned chunks small enough for a call of npairs pairs.
+int fast64_threads(int compute_tau);   // default block size
+void deposit_fit_chunk(DepositLaunch &cfg, long long npairs, int sms);
+size_t deposit_split_bytes(const DepositLaunch &cfg, int nbins, int nlos, int sms);
 // CTAs of the deposit kernel that fit on one SM for this configuration.
 int deposit_resident_ctas(const DepositLaunch &cfg, int compute_tau, int nbins);
 // Plain FP64 atomics into out for the listed lines (non-finite propagation).

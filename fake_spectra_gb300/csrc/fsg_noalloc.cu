@@ -305,7 +305,7 @@ int noalloc_run(int compute_tau, int nbins, int kernel, double box, double velfa
         cfg.tiles = 1;
         cfg.fast64 = precision == FSG_PREC_FP64;
         if (cfg.fast64) {
-            cfg.threads = 512;
+            cfg.threads = fast64_threads(compute_tau);
             deposit_plan(cfg, compute_tau, nbins);
             if (!cfg.smem_mode) {   // no room beside the accumulators: the direct walk
                 cfg.fast64 = 0;
@@ -317,11 +317,14 @@ int noalloc_run(int compute_tau, int nbins, int kernel, double box, double velfa
         cfg.persistent = precision == FSG_PREC_FP32 || cfg.fast64 ? 1 : 0;
         int sms = 0;
         NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
-        if (cfg.fast64) {
-            deposit_clusters(cfg, compute_tau, nbins, nlos);
-        } else {
-            const int per_sm = std::max(1, deposit_resident_ctas(cfg, compute_tau, nbins));
-            cfg.grid = std::min(nlos, sms * per_sm);
+        const int per_sm = std::max(1, deposit_resident_ctas(cfg, compute_tau, nbins));
+        cfg.grid = std::min(nlos, sms * per_sm);
+        // the scratch behind the dr2 values in use can hold the state of shared sightlines
+        deposit_fit_chunk(cfg, total, sms);
+        const size_t sb = deposit_split_bytes(cfg, nbins, nlos, sms);
+        if (sb && (size_t)(pair_cap - total) * 8 >= sb + 256) {
+            cfg.split_ws = (void *)(((uintptr_t)(d_dr2 + total) + 255) & ~(uintptr_t)255);
+            cfg.grid = sms * per_sm;
         }
         PairLists pl{d_off, d_part, d_dr2};
         NA_CUDA(cudaMemsetAsync(d_ticket, 0, 4, s), "memset");

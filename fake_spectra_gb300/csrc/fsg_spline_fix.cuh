@@ -19,15 +19,6 @@
 
 namespace fsg {
 
-FSG_HD int fix_clz64(uint64_t v)   // v != 0
-{
-#ifdef __CUDA_ARCH__
-    return __clzll((long long)v);
-#else
-    return __builtin_clzll(v);
-#endif
-}
-
 // q = sqrt(s), units of 2^-64, s >= 2^-16: error below 2^-61.
 FSG_HD uint64_t fix_sqrt64_upper(uint64_t s)
 {

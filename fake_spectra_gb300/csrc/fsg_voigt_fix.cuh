@@ -158,10 +158,10 @@ FSG_HD void fix_node_sums(const FixPair &p, int64_t V, const Rows &rows, const F
             const uint64_t x2 = fix_umulhi64(x << 8, x << 8);      // 2^-58
             const uint32_t x2h = (uint32_t)(x2 >> 32);             // 2^-26
             const uint32_t x4 = (uint32_t)(((uint64_t)x2h * x2h) >> 32);   // 2^-20
-            const uint32_t x6 = (uint32_t)(((uint64_t)x4 * x2h) >> 32);    // 2^-14
             uint64_t y = fix_umulhi64(x2, p.k1);                   // 2^-57
             y += ((uint64_t)x4 * (uint32_t)p.k2) >> 20;
-            y += ((uint64_t)x6 * (uint32_t)p.k3) >> 24;
+            if (p.k3)
+                y += ((uint64_t)(uint32_t)(((uint64_t)x4 * x2h) >> 32) * (uint32_t)p.k3) >> 24;
             const int n = (int)(y >> 57);
             const int k = (int)(y >> 51) & 63;
             const Fix62 r = fix62(y << 13);
@@ -255,6 +255,173 @@ inline
     p.sal -= 32;         // the product drops its low 32 bits first
     // a^4 K''''/120: K''''/24 = d4 2^24 / (2h)^4
     fix_mantissa(a2 * a2 / 5.0 * 65536.0 * 16777216.0, p.be, p.sbe);
+}
+
+// ------------------------------------------------------------- numbers m 2^e
+FSG_HD int fix_clz64(uint64_t v)   // v != 0
+{
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)v);
+#else
+    return __builtin_clzll(v);
+#endif
+}
+
+FSG_HD uint64_t fix_bits(double d)
+{
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(d);
+#else
+    uint64_t u;
+    __builtin_memcpy(&u, &d, 8);
+    return u;
+#endif
+}
+
+FSG_HD double fix_from_bits(uint64_t u)
+{
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)u);
+#else
+    double d;
+    __builtin_memcpy(&d, &u, 8);
+    return d;
+#endif
+}
+
+// A positive normal double as m 2^e, m in [2^63, 2^64).
+struct FixNum {
+    uint64_t m;
+    int e;
+};
+FSG_HD FixNum fix_num(double d)
+{
+    const uint64_t u = fix_bits(d);
+    FixNum r;
+    r.m = (u << 11) | (1ull << 63);
+    r.e = (int)((u >> 52) & 0x7FF) - 1086;
+    return r;
+}
+
+// m 2^e as a double (the result must be normal; m = 0 gives 0), sign bit `neg`.
+FSG_HD double fix_double(uint64_t m, int e, uint64_t neg)
+{
+    if (m == 0)
+        return 0.0;
+    const int lz = fix_clz64(m);
+    const uint64_t n = m << lz;
+    const uint64_t r = (n >> 11) + ((n >> 10) & 1ull);   // 53 bits, bit 52 set (or a carry)
+    return fix_from_bits((neg << 63) | ((((uint64_t)(e + 1085 - lz)) << 52) + r));
+}
+
+// A velocity in units of b from twice its value: |V| = p 2^(-53 - s), p in
+// [2^62, 2^64); ib, eb: 1/b = ib 2^eb.
+struct FixV {
+    uint64_t p;
+    int s;
+};
+FSG_HD FixV fix_velocity(double v2, uint64_t ib, int eb)
+{
+    const uint64_t u = fix_bits(v2);
+    const int E = (int)((u >> 52) & 0x7FF);
+    FixV r;
+    r.p = fix_umulhi64((u << 11) | (1ull << 63), ib);
+    r.s = 970 - E - eb;       // v2 = 0: E = 0, a shift beyond the word
+    return r;
+}
+// |V| in units of 2^-53 (saturating)
+FSG_HD uint64_t fix_v53(FixV v)
+{
+    return v.s < 0 ? 0x7FFFFFFFFFFFFFFFull : (v.s > 63 ? 0ull : v.p >> v.s);
+}
+
+// 1 / (p 2^-64) for p in [2^63, 2^64), units of 2^-63 (error below 2^-61): the
+// float reciprocal and one third-order Newton step.
+FSG_HD uint64_t fix_recip(uint64_t p)
+{
+    const float pf = (float)(uint32_t)(p >> 32);
+#ifdef __CUDA_ARCH__
+    const uint32_t r0 = __float2uint_rz(fminf(9223372036854775808.0f * __frcp_rn(pf),
+                                              4294967040.0f));
+#else
+    const float rf = 9223372036854775808.0f / pf;
+    const uint32_t r0 = (uint32_t)(rf < 4294967040.0f ? rf : 4294967040.0f);
+#endif
+    // e = 1 - r0 p, units of 2^-63
+    const uint64_t t = (p >> 32) * r0 + (((p & 0xFFFFFFFFull) * r0) >> 32);
+    const int64_t e1 = (int64_t)((1ull << 63) - t);
+    const int64_t e12 = e1 >> 12;
+    const int64_t d = e1 + ((e12 * e12) >> 39);
+    const int64_t dh = d >> 32;
+    const uint64_t dl = (uint64_t)d & 0xFFFFFFFFull;
+    return ((uint64_t)r0 << 32) + (uint64_t)(dh * (int64_t)r0 * 2) + ((dl * r0) >> 31);
+}
+
+// Far wing: A_1 y + A_2 y^2 + ..., y = (vmp / V)^2 < 1, as cA y times the sum of
+// (A_r / A_1) y^(r-1).
+constexpr int FIX_FAR_R = 16;
+struct FixFar {
+    uint64_t vs, cA;         // vmp^2 = vs 2^ev; scale A_1 = cA 2^eA
+    int32_t ev, eA;
+    int64_t A[FIX_FAR_R - 1];   // A_(r+1) / A_1 2^r, units of 2^-61
+};
+
+// y = ym 2^ye of a velocity beyond vmp, ym in [2^63, 2^64)
+FSG_HD uint64_t fix_far_y(const FixFar &f, FixV v, int &ye)
+{
+    const int lz = (int)(~v.p >> 63);
+    const uint64_t r = fix_recip(v.p << lz);
+    const uint64_t m = fix_umulhi64(fix_umulhi64(r, r), f.vs);
+    const int lm = fix_clz64(m);
+    ye = f.ev - 20 + 2 * (v.s + lz) - lm;    // -126 - 2 q + ev, q = -53 - s - lz
+    return m << lm;
+}
+
+// The wing's value m 2^e from n >= 2 terms (from the eighth on the upper half of y
+// is enough).
+FSG_HD uint64_t fix_far_sum(const FixFar &f, int n, uint64_t ym, int ye, int &e)
+{
+    const int sh = -64 - ye;                 // y 2^64 = ym >> sh
+    const Fix62 y = fix62(sh > 63 ? 0ull : ym >> sh);
+    int64_t acc = f.A[n - 2];
+    int r = n - 3;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+    for (; r >= 6; r--)
+        acc = fix_fma_hi(acc, y.hi, f.A[r]);
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+    for (; r >= -1; r--)
+        acc = fix_fma(acc, y, r >= 0 ? f.A[r] : (int64_t)1 << 61);
+    const uint64_t m1 = fix_umulhi64((uint64_t)acc << 2, ym);
+    e = 65 + f.eA + ye;
+    return fix_umulhi64(m1, f.cA);
+}
+
+// sg 2^(-60 - eg) cg + sk 2^(-60 - ek) ck as m 2^e (a positive sum).
+FSG_HD uint64_t fix_combine(int64_t sg, int eg, FixNum cg, int64_t sk, int ek, FixNum ck, int &e)
+{
+    uint64_t gm = 0, km = 0;
+    int xg = -100000, xk = -100000;
+    if (sg > 0) {
+        const int lz = fix_clz64((uint64_t)sg);
+        gm = fix_umulhi64((uint64_t)sg << lz, cg.m) >> 2;   // room for the sum
+        xg = 6 - lz + cg.e - eg;
+    }
+    if (sk != 0) {
+        const uint64_t a = (uint64_t)(sk < 0 ? -sk : sk);
+        const int lz = fix_clz64(a);
+        km = fix_umulhi64(a << lz, ck.m) >> 2;
+        xk = 6 - lz + ck.e - ek;
+    }
+    e = xg > xk ? xg : xk;
+    const int dg = e - xg, dk = e - xk;
+    gm = dg > 63 ? 0ull : gm >> dg;
+    km = dk > 63 ? 0ull : km >> dk;
+    const int64_t t = (int64_t)gm + (sk < 0 ? -(int64_t)km : (int64_t)km);
+    return t > 0 ? (uint64_t)t : 0ull;
 }
 
 }  // namespace fsg
