@@ -845,7 +845,7 @@ fsg_tune_entry tune_deposit(fsg_context *c, const LineParams &lp, const Particle
                  {1024, 8, 1, 0}, {1024, 16, 1, 0}, {1024, 8, 1, 1}, {768, 8, 1, 1}};
     else
         cands = {{512, 32, 1, 0}, {512, 16, 1, 0}, {512, 8, 1, 0}, {512, 32, 0, 0},
-                 {256, 32, 1, 0}, {256, 16, 1, 0}};
+                 {256, 32, 1, 0}, {256, 16, 1, 0}, {1024, 16, 1, 0}, {1024, 8, 1, 0}};
     fsg_tune_entry best{};
     best.ms_best = 1e300;
     best.sample_lines = nsamp;

@@ -1043,17 +1043,16 @@ struct Bound32 {
 
 // tau_pair_bound in FP32 arithmetic with a 1e-3 margin (the FP32 form's
 // contributions are FP32 values too): no FP64 work per pair beyond the overlap
-// test, which follows the reference's double comparison.
-__device__ __forceinline__ double tau_pair_bound32(const Bound32 &k, const PairInput &in)
+// test, the reference's double comparison hh2 <= dr2 (hh2 is a float, so the
+// float below dr2 decides it).
+__device__ __forceinline__ float tau_pair_bound32(const Bound32 &k, const PairInput &in)
 {
-    const double hh2 = (double)__fmul_rn(in.smooth, in.smooth);
-    if (hh2 - in.dr2 <= 0)
-        return 0.0;
+    if (__double2float_rd(in.dr2) >= __fmul_rn(in.smooth, in.smooth))
+        return 0.f;
     const float btherm = k.bfac * sqrtf(in.temp);
     const float aa = k.voigt_fac / btherm;
     const float hmax = aa >= 0.f ? 1.f : 2.f * expf(aa * aa) + 1.f;
-    return (double)(fabsf(k.ampc / btherm * in.dens) * (k.velfac_abs * fabsf(in.smooth)) *
-                    k.kfac * hmax);
+    return fabsf(k.ampc / btherm * in.dens) * (k.velfac_abs * fabsf(in.smooth)) * k.kfac * hmax;
 }
 
 // Upper bound of |taulast| for a pair (any pixel): |amp dens/velfac| x deltav x
@@ -1178,6 +1177,46 @@ __device__ __forceinline__ double colden_pair_bound(const LineParams &lp, const 
            (wraps > 1.0 ? wraps : 1.0);
 }
 
+// kern_frac of the pixel [plow, plow + pixel) clipped to the kernel support, for
+// the FP32 form's end pixels, in integer arithmetic (fix_spline_sum; FP64 runs
+// at 1/64 of the FP32 rate, and the two end pixels of every pair took 18 FP64
+// square roots and divisions: 28.6 ms for 1.0e7 pairs, 23.6 ms so).  The
+// value agrees with the double one to about 2^-53 / (1 - q), far below the float
+// it is rounded to; pairs that graze the support (zrange < h / 64), where it
+// would not be, and the kernels without a square root keep the double form.
+struct ColdenEnds {
+    bool fix, cubic;
+    double inv_h;            // 2^62 / h
+    uint64_t B;              // dr2 / h^2, units of 2^-64
+    __device__ __forceinline__ explicit ColdenEnds(const Colden &c)
+    {
+        cubic = c.kernel == SPH_CUBIC;
+        const double h2 = c.smooth * c.smooth;
+        fix = (cubic || c.kernel == SPH_QUINTIC) && c.zrange * c.zrange * 4096.0 > h2 &&
+              h2 < 1e200 && h2 > 1e-200 && c.zrange <= c.smooth;
+        const double inv = 1.0 / c.smooth;
+        inv_h = 4611686018427387904.0 * inv;
+        B = fix ? __double2ull_rn(c.dr2 * inv * inv * 18446744073709551616.0) : 0ull;
+    }
+    __device__ __forceinline__ double value(const Colden &c, long long z) const
+    {
+        double plow = __dsub_rn(__dmul_rn(c.boxtokpc, (double)z), c.pos1);
+        double phigh = __dadd_rn(plow, c.boxtokpc);
+        if (!fix)
+            return kern_frac<double>(c.kernel, plow, phigh, c.smooth, c.dr2, c.zrange);
+        plow = fmax(plow, -c.zrange);
+        phigh = fmin(phigh, c.zrange);
+        if (plow > phigh)
+            return 0.0;
+        int e;
+        const int64_t sum = fix_spline_sum<true>(cubic, __double2ll_rn(plow * inv_h),
+                                                 __double2ll_rn(phigh * inv_h), B, e);
+        const double norm = cubic ? 32. / 4 / PI_D : 9. / 40 / PI_D * 243.0;
+        return scalbn((phigh - plow) * norm * __ll2double_rn(sum),
+                      -(62 + (cubic ? 3 : 5) * e));
+    }
+};
+
 // Per-pair constants of the FP32 column density (48 bytes), set up by one
 // lane per pair like Stage32: the three FP64 edge pixels (first, last two)
 // are evaluated here, lane-parallel, and the interior walks in FP32.
@@ -1208,9 +1247,16 @@ __device__ __forceinline__ void stagecol32_setup(const LineParams &lp, const Pai
     st.j0 = wrap_bin(c.zlow, lp.nbins);
     st.kmax = (int)c.kmax;
     st.dens_f = c.dens_f;
-    st.e0 = (float)c.value64(c.zlow);
-    st.e1 = c.kmax >= 2 ? (float)c.value64(c.zlow + c.kmax - 1) : 0.f;
-    st.e2 = c.kmax >= 1 ? (float)c.value64(c.zhigh) : 0.f;
+    const ColdenEnds ends(c);
+    float v[3];
+#pragma unroll 1
+    for (int i = 0; i < 3; i++)   // pixels 0, kmax - 1 and kmax, where they differ
+        v[i] = c.kmax >= (3 - i) % 3
+                   ? (float)__dmul_rn(c.dens, ends.value(c, c.zlow + (i ? c.kmax - 2 + i : 0)))
+                   : 0.f;
+    st.e0 = v[0];
+    st.e1 = v[1];
+    st.e2 = v[2];
     st.dL0 = c.dL0;
     st.dR0 = c.dR0;
     st.two_zr = c.two_zr;
@@ -1239,18 +1285,24 @@ __device__ __forceinline__ float colden_interior32(const StageCol32 &st, int ker
     return st.dens_f * (dz * total);
 }
 
-// colden_pair_bound in FP32 with a 1e-3 margin: the window length is bounded
-// by 2 zrange / pixel + 3 pixels.
-__device__ __forceinline__ double colden_pair_bound32(const LineParams &lp, const PairInput &in,
-                                                      float btk_abs, float kfac)
+// Windows of the row a pair covers (1 at least), from the window length 2 zrange /
+// pixel + 3 pixels; 0 for a pair that misses the sightline.
+__device__ __forceinline__ float colden_wraps32(const LineParams &lp, const PairInput &in,
+                                                float btk_abs)
 {
-    const double hh2 = (double)__fmul_rn(in.smooth, in.smooth);
-    if (hh2 - in.dr2 <= 0)
-        return 0.0;
-    const float zr = sqrtf((float)(hh2 - in.dr2));
-    const float npix = 2.f * zr / btk_abs + 3.f;
-    const float wraps = fmaxf(1.f, ceilf(npix / (float)lp.nbins));
-    return (double)(fabsf(in.dens) * kfac * btk_abs * wraps);
+    const float d = (float)((double)__fmul_rn(in.smooth, in.smooth) - in.dr2);
+    if (d <= 0.f)
+        return 0.f;
+    const float npix = 2.f * sqrtf(d) / btk_abs + 3.f;
+    return fmaxf(1.f, ceilf(npix / (float)lp.nbins));
+}
+
+// colden_pair_bound in FP32 with a 1e-3 margin.
+__device__ __forceinline__ float colden_pair_bound32(const LineParams &lp, const PairInput &in,
+                                                     float btk_abs, float kfac)
+{
+    const float wraps = colden_wraps32(lp, in, btk_abs);
+    return wraps == 0.f ? 0.f : fabsf(in.dens) * kfac * btk_abs * wraps;
 }
 
 // ------------------------------------------------------------ reductions
@@ -1270,6 +1322,33 @@ struct BoundScratch {
     unsigned long long q[32];
 };
 
+// A bound's finiteness, its ilogb and ceil(b 2^s) (b > 0, the result below 2^31);
+// for float bounds on the bits, without FP64 work.
+__device__ __forceinline__ bool bound_finite(double b) { return isfinite(b); }
+__device__ __forceinline__ bool bound_finite(float b)
+{
+    return (__float_as_uint(b) & 0x7F800000u) != 0x7F800000u;
+}
+__device__ __forceinline__ int bound_ilogb(double b) { return ilogb(b); }
+__device__ __forceinline__ int bound_ilogb(float b)
+{
+    const unsigned u = __float_as_uint(b);
+    return u >= 0x800000u ? (int)(u >> 23) - 127 : -118 - __clz((int)u);
+}
+__device__ __forceinline__ unsigned long long bound_units(double b, int s)
+{
+    return (unsigned long long)ceil(scalbn(b, s));
+}
+__device__ __forceinline__ unsigned long long bound_units(float b, int s)
+{
+    const unsigned u = __float_as_uint(b), e = u >> 23;
+    const unsigned m = (u & 0x7FFFFFu) | (e ? 0x800000u : 0u);
+    const int k = (int)(e ? e : 1u) - 150 + s;   // b 2^s = m 2^k, k <= 7
+    if (k >= 0)
+        return (unsigned long long)m << k;
+    return k > -32 ? ((unsigned long long)m + (1ull << -k) - 1ull) >> -k : 1ull;
+}
+
 template <class BoundFn, class AgainFn>
 __device__ __forceinline__ double order_free_bound(long long e0, long long e1, BoundFn bound,
                                                    AgainFn bound_again, BoundScratch *sc)
@@ -1279,11 +1358,11 @@ __device__ __forceinline__ double order_free_bound(long long e0, long long e1, B
     int em = NONE;
     bool bad = false;
     for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        const double b = bound(e);
-        if (!isfinite(b))
+        const auto b = bound(e);
+        if (!bound_finite(b))
             bad = true;
-        else if (b > 0.0)
-            em = max(em, ilogb(b));
+        else if (b > 0)
+            em = max(em, bound_ilogb(b));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -1302,9 +1381,9 @@ __device__ __forceinline__ double order_free_bound(long long e0, long long e1, B
         return 0.0;
     unsigned long long q = 0;
     for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        const double b = bound_again(e);
-        if (b > 0.0)
-            q += (unsigned long long)ceil(scalbn(b, 30 - eall));
+        const auto b = bound_again(e);
+        if (b > 0)
+            q += bound_units(b, 30 - eall);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -2128,8 +2207,103 @@ __device__ __forceinline__ PairInput load_pair_ch(const ChannelArgs &a, long lon
     return load_pair(p, a.pl, e, axis, false, a.dev_err);
 }
 
+// order_free_bound of every channel over the pairs [e0, e1) (whole block): the
+// same values, exponents and integer sums, with two passes over the pairs in all
+// instead of two per channel.
 template <int PREC>
-__global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(ChannelArgs a)
+__device__ void channel_bounds(const ChannelArgs &a, int axis, long long e0, long long e1,
+                               double btk, float btk_abs, float col_kfac, BoundScratch *sc,
+                               double *B, int *bad)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int NONE = -2147483647, INF = 2147483647;
+    int em[MAX_CHANNELS], eall[MAX_CHANNELS];
+    unsigned long long q[MAX_CHANNELS];
+    // f(c, bound) for every pair of this thread and channel
+    const auto each = [&](auto f) {
+        for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+            PairInput in = load_pair_ch(a, e, axis, 0);
+            const int ip = a.pl.part[e];
+            const bool named = (unsigned long long)(long long)ip < (unsigned long long)a.p.n;
+            // the channel's bound is its density times this, in the single form's order
+            in.dens = 1.f;
+            typename std::conditional<PREC == 1, float, double>::type wraps = 0;
+            if constexpr (PREC == 1) {
+                wraps = colden_wraps32(a.lp, in, btk_abs);
+            } else {
+                Colden c;
+                if (c.setup(a.lp, in, btk)) {
+                    const double w = ceil((double)(c.zhigh - c.zlow + 1) / a.lp.nbins);
+                    wraps = w > 1.0 ? w : 1.0;
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < MAX_CHANNELS; c++)
+                if (c < a.nch) {
+                    const float d = named ? __ldg(&a.dens[c][ip]) : 0.f;
+                    auto b = wraps;   // 0: the pair misses the sightline
+                    if (wraps != 0) {
+                        if constexpr (PREC == 1)
+                            b = fabsf(d) * col_kfac * btk_abs * wraps;
+                        else
+                            b = fabs((double)d) * kernel_max(a.lp.kernel) * fabs(btk) * 1.001 *
+                                wraps;
+                    }
+                    f(c, b);
+                }
+        }
+    };
+#pragma unroll
+    for (int c = 0; c < MAX_CHANNELS; c++) {
+        em[c] = NONE;
+        q[c] = 0ull;
+    }
+    each([&](int c, auto b) {
+        em[c] = !bound_finite(b) ? INF : (b > 0 ? max(em[c], bound_ilogb(b)) : em[c]);
+    });
+#pragma unroll
+    for (int c = 0; c < MAX_CHANNELS; c++) {
+        eall[c] = NONE;
+        if (c < a.nch) {
+            const int m = __reduce_max_sync(0xffffffffu, em[c]);
+            __syncthreads();
+            if (lane == 0)
+                sc->em[warp] = m;
+            __syncthreads();
+            for (int i = 0; i < nw; i++)
+                eall[c] = max(eall[c], sc->em[i]);
+        }
+    }
+    each([&](int c, auto b) {
+        if (b > 0 && eall[c] != INF)
+            q[c] += bound_units(b, 30 - eall[c]);
+    });
+#pragma unroll
+    for (int c = 0; c < MAX_CHANNELS; c++)
+        if (c < a.nch) {
+            unsigned long long v = q[c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                v += __shfl_xor_sync(0xffffffffu, v, o);
+            __syncthreads();
+            if (lane == 0)
+                sc->q[warp] = v;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                unsigned long long Q = 0;
+                for (int i = 0; i < nw; i++)
+                    Q += sc->q[i];
+                B[c] = eall[c] == INF ? __longlong_as_double(0x7ff0000000000000ll)
+                                      : (eall[c] == NONE ? 0.0
+                                                         : scalbn(__ull2double_ru(Q), eall[c] - 30));
+                bad[c] = eall[c] == INF;
+            }
+        }
+    __syncthreads();
+}
+
+template <int PREC>
+__global__ void __launch_bounds__(PREC == 0 ? 256 : 512, 1) colden_channels_kernel(ChannelArgs a)
 {
     extern __shared__ __align__(16) unsigned long long smem[];
     __shared__ BoundScratch red;
@@ -2157,19 +2331,9 @@ __global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(
         const int line = a.line_order[ticket];
         const int axis = a.t.axis[line];
         const long long e0 = a.pl.off[line], e1 = a.pl.off[line + 1];
-        // 1. per-channel bounds, summed exactly as the single-channel deposit sums them
-        for (int c = 0; c < nch; c++) {
-            const auto bf = [&](long long e) {
-                const PairInput in = load_pair_ch(a, e, axis, c);
-                return PREC == 1 ? colden_pair_bound32(a.lp, in, btk_abs, col_kfac)
-                                 : colden_pair_bound(a.lp, in, btk);
-            };
-            const double B = order_free_bound(e0, e1, bf, bf, &red);
-            if (threadIdx.x == 0) {
-                s_B[c] = B;
-                s_bad[c] = !isfinite(B);
-            }
-        }
+        // 1. per-channel bounds, summed exactly as the single-channel deposit sums
+        // them; a pair's geometry is formed once for all channels
+        channel_bounds<PREC>(a, axis, e0, e1, btk, btk_abs, col_kfac, &red, s_B, s_bad);
         for (size_t j = threadIdx.x; j < acc_words; j += blockDim.x)
             acc[j] = 0ull;
         if (threadIdx.x == 0)
@@ -2212,14 +2376,14 @@ __global__ void __launch_bounds__(PREC == 0 ? 256 : 512) colden_channels_kernel(
                 } else {
                     st.j0 = wrap_bin(col.zlow, nbins);
                     st.kmax = (int)col.kmax;
-                    const auto kf = [&](long long z) {
-                        const double plow = __dsub_rn(__dmul_rn(btk, (double)z), col.pos1);
-                        return kern_frac<double>(a.lp.kernel, plow, __dadd_rn(plow, btk), col.smooth,
-                                                 col.dr2, col.zrange);
-                    };
-                    st.kf0 = kf(col.zlow);
-                    st.kf1 = col.kmax >= 2 ? kf(col.zlow + col.kmax - 1) : 0.0;
-                    st.kf2 = col.kmax >= 1 ? kf(col.zhigh) : 0.0;
+                    const ColdenEnds ends(col);
+                    st.kf0 = st.kf1 = st.kf2 = 0.0;
+#pragma unroll 1
+                    for (int i = 0; i < 3; i++)
+                        if (col.kmax >= (3 - i) % 3) {
+                            const double f = ends.value(col, col.zlow + (i ? col.kmax - 2 + i : 0));
+                            (i == 0 ? st.kf0 : (i == 1 ? st.kf1 : st.kf2)) = f;
+                        }
                     st.dL0 = col.dL0;
                     st.dR0 = col.dR0;
                     st.two_zr = col.two_zr;

@@ -52,7 +52,9 @@ FSG_HD uint64_t fix_sqrt64(uint64_t s)
 
 // Trapezoid sum over the 9 nodes from z = za to zb (units of 2^-62 of h) of the
 // cubic (W / (8/pi)) or quintic (W / (9/(40 pi)) / 243) kernel, B = dr2 / h^2 in
-// units of 2^-64.  The sum is (return value) 2^(-59 - 3e) or 2^(-59 - 5e).
+// units of 2^-64.  The sum is (return value) 2^(-59 - 3e) or 2^(-59 - 5e).  EDGE:
+// nodes may reach q >= 1, where the kernel is zero.
+template <bool EDGE = false>
 FSG_HD int64_t fix_spline_sum(bool cubic, int64_t za, int64_t zb, uint64_t B, int &e)
 {
     const uint64_t ua = (uint64_t)(za < 0 ? -za : za), ub = (uint64_t)(zb < 0 ? -zb : zb);
@@ -91,6 +93,8 @@ FSG_HD int64_t fix_spline_sum(bool cubic, int64_t za, int64_t zb, uint64_t B, in
             if (t > 2 * third)
                 w += 15 * pow5((t - 2 * third) << e);
         }
+        if (EDGE && s < B)
+            w = 0;
         sum += (j == 0 || j == 8) ? w >> 1 : w;
     }
     return sum;
