@@ -1053,8 +1053,7 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
     }
     cuda_check(cudaEventRecord(c->ev[2], s), "event");
     cuda_check(cudaGraphLaunch(c->graph, s), "graph launch");
-    for (const DepositLaunch &cf : cfgs)   // deposit, fallback (+ tile weights)
-        c->stats.gpu_launches += 2 + (nlos > 0 && cf.tiles && !cf.fast64 ? 1 : 0);
+    c->stats.gpu_launches += 2 * (long long)cfgs.size();   // deposit, fallback
     cuda_check(cudaEventRecord(c->ev[3], s), "event");
     unsigned h_err = 0;
     cuda_check(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "read");
@@ -1627,10 +1626,13 @@ static int tau_backward(fsg_context *ctx, const unsigned long long *reuse_gen, i
         cuda_check(cudaMemsetAsync(err, 0, sizeof(unsigned), s), "memset");
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-        const int grid = std::min(nlos, sms * std::max(1, tau_backward_resident_ctas()));
+        const int grid = std::min(nlos, sms * std::max(1, tau_backward_resident_ctas(nbins)));
+        const size_t row = tau_backward_row_bytes(nbins);
+        float *rows = row ? (float *)ctx->ensure(ctx->gacc, row * grid) : nullptr;
         cuda_check(cudaEventRecord(ctx->ev[2], s), "event");
         launch_tau_backward(lp, ctx->tables, p, pl, (const int *)ctx->line_order.p, nlos,
-                            grad_tau, grad_dens, grad_temp, grad_vel, ticket, err, grid, s);
+                            grad_tau, grad_dens, grad_temp, grad_vel, ticket, err, rows, grid,
+                            s);
         ctx->stats.gpu_launches++;
         cuda_check(cudaGetLastError(), "backward launch");
         cuda_check(cudaEventRecord(ctx->ev[3], s), "event");

@@ -709,7 +709,8 @@ static_assert(sizeof(Stage32) == 80, "Stage32 is five 16-byte words");
 // SingleAbsorber (singleabs.h:81-90) and the per-particle constants of
 // add_tau_particle (absorption.cpp:225-247), FP32 form.  Returns false for a
 // pair whose smoothing sphere misses the sightline (absorption.cpp:232).
-// scale_nod (may be null) receives scale without the density factor.
+// scale_nod (may be null) receives scale without the density factor, dcoef (may
+// be null) the far-wing coefficients of the temperature derivative.
 // Float copies of the line constants the FP32 setup uses (once per sightline).
 struct Setup32 {
     float bfac, voigt_fac, ampv, bintov;   // ampv = sigma_a / sqrt(pi) c / velfac
@@ -730,7 +731,8 @@ struct Setup32 {
 // within 4e-7 of the double one).
 __device__ __forceinline__ bool stage32_setup(const LineParams &lp, const Setup32 &k,
                                               const PairInput &in, double bintov_d,
-                                              Stage32 &st, float *scale_nod)
+                                              Stage32 &st, float *scale_nod,
+                                              float *dcoef = nullptr)
 {
     const double hh2 = (double)__fmul_rn(in.smooth, in.smooth);
     if (hh2 - in.dr2 <= 0)
@@ -783,6 +785,24 @@ __device__ __forceinline__ bool stage32_setup(const LineParams &lp, const Setup3
             for (int j = 1; j <= r; j++)
                 acc = fmaf(gam[j] * binom_f(2 * r - 1, 2 * r - 2 * j), M[r - j], acc);
             st.A[r - 1] = acc;
+        }
+        if (dcoef) {
+            // the backward kernel's sum of H + u dH/du + a dH/da: a term of degree
+            // n in (U, V, a) together takes the factor 1 + n (1 - 2j for a u^-2j,
+            // 3 - 2j for a^3 u^-2j)
+#pragma unroll
+            for (int j = 1; j <= MP_R; j++)
+                gam[j] = vc.a_sqpi * ((float)(2 - 2 * j) * P[j - 1] -
+                                      (j >= 2 && j - 2 < 5
+                                           ? (float)(4 - 2 * j) * vc.a2 * Q[j - 2] : 0.f));
+#pragma unroll
+            for (int r = 1; r <= MP_R; r++) {
+                float acc = 0.f;
+#pragma unroll
+                for (int j = 1; j <= r; j++)
+                    acc = fmaf(gam[j] * binom_f(2 * r - 1, 2 * r - 2 * j), M[r - j], acc);
+                dcoef[r - 1] = acc;
+            }
         }
         const float umax = 3.f * fabsf(st.u1);
         st.vmp = fmaxf(3.34f * umax, umax + 6.5f);
@@ -1602,45 +1622,35 @@ constexpr int TILE_W = 64;
 constexpr int TILE_M = 8;
 constexpr float TILE_DIST = 128.f;
 
-__device__ double g_tile_w[TILE_W * TILE_M];   // [pixel in tile][node] interpolation weights
-__device__ float g_tile_x[TILE_M];             // node positions, pixels from the tile's first
-
-// Node positions x_k = 31.5 (1 + cos((2k+1) pi / 2M)) rounded to float, and
-// the barycentric Lagrange weights of those float positions at the pixels.
-__global__ void tile_weights_kernel()
+// Node positions x_k = 31.5 (1 + cos((2k+1) pi / 2M)) as floats, pixels from the
+// tile's first, and the barycentric Lagrange weights of those positions at the
+// tile's pixels, [pixel in tile][node].
+struct TileTables {
+    float x[TILE_M];
+    double w[TILE_W * TILE_M];
+};
+constexpr TileTables tile_tables()
 {
-    const int t = threadIdx.x;
-    if (t >= TILE_W * TILE_M)
-        return;
-    const int p = t / TILE_M, k = t % TILE_M;
-    const double h = 0.5 * (TILE_W - 1);
-    double x[TILE_M];
-#pragma unroll
-    for (int i = 0; i < TILE_M; i++)
-        x[i] = (double)(float)(h + h * cos((2 * i + 1) * PI_D / (2 * TILE_M)));
-    double num = 0.0, den = 0.0;
-    bool hit = false;
-#pragma unroll
+    TileTables t{{62.394737243652344f, 57.69129180908203f, 49.00046157836914f, 37.64534378051758f,
+                  25.35465431213379f, 13.999537467956543f, 5.308707237243652f,
+                  0.6052636504173279f}, {}};
+    double lam[TILE_M] = {};
     for (int i = 0; i < TILE_M; i++) {
-        double lam = 1.0;
-#pragma unroll
+        lam[i] = 1.0;
         for (int j = 0; j < TILE_M; j++)
             if (j != i)
-                lam /= (x[i] - x[j]);
-        const double d = (double)p - x[i];
-        if (d == 0.0) {
-            hit = true;
-            num = (i == k) ? 1.0 : 0.0;
-            break;
-        }
-        den += lam / d;
-        if (i == k)
-            num = lam / d;
+                lam[i] /= (double)t.x[i] - (double)t.x[j];
     }
-    g_tile_w[t] = hit ? num : num / den;
-    if (p == 0)
-        g_tile_x[k] = (float)x[k];
+    for (int p = 0; p < TILE_W; p++) {   // no node falls on a pixel
+        double den = 0.0;
+        for (int i = 0; i < TILE_M; i++)
+            den += lam[i] / ((double)p - (double)t.x[i]);
+        for (int k = 0; k < TILE_M; k++)
+            t.w[p * TILE_M + k] = lam[k] / ((double)p - (double)t.x[k]) / den;
+    }
+    return t;
 }
+__device__ const TileTables g_tile = tile_tables();
 
 // |V| (in units of b) where the far wing equals tautail: the root of
 // h(W) = sum_r A_r W^(r+1) = tautail in W = 1/V^2.  h is increasing and convex
@@ -1736,7 +1746,7 @@ __device__ __forceinline__ void walk_tau32_tiled(const DepositArgs &a, const Tau
                 const int t = it / TILE_M, m = it - t * TILE_M;
                 const int kt = k + TILE_W * t;
                 ka = (float)(dir == 0 ? kt : -kt - TILE_W);
-                kb = g_tile_x[m];
+                kb = g_tile.x[m];
                 idx = (dir == 0 ? jb_run + TILE_W * t : jb_run - TILE_W * (t + 1) + 1) / TILE_W *
                           TILE_M + m;
             } else {
@@ -2068,7 +2078,7 @@ __global__ void __launch_bounds__(MAXT, 1)
                 for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
                     double v = from_split(lo[j], hi[j], S);
                     if (j < ntiles * TILE_W) {
-                        const double *w = g_tile_w + (j % TILE_W) * TILE_M;
+                        const double *w = g_tile.w + (j % TILE_W) * TILE_M;
                         const double *nd = node + (j / TILE_W) * TILE_M;
                         double f = 0.0;
 #pragma unroll
@@ -2507,6 +2517,7 @@ struct GradArgs {
     float *g_dens, *g_temp, *g_vel;
     unsigned *ticket;
     unsigned *dev_err;
+    float *rows;             // per block, rows too long for shared memory; else null
 };
 
 struct GradSums {
@@ -2615,72 +2626,159 @@ __device__ __noinline__ void grad_pair_careful(const GradArgs &a, const PairInpu
 }
 
 // Staged pair of the backward kernel: the forward constants plus what the
-// gradient needs (96 bytes).
+// gradient needs (128 bytes).
 struct __align__(16) StageGrad {
     Stage32 s;
+    float D[MP_R];           // far-wing coefficients of the temperature derivative
     float scale_nod, temp;
     int ip, pad;
 };
-// 1024 threads at 64 registers (32 warps per SM; the kernel spills the same
-// ~250 bytes at 128 registers), 16 staged pairs per warp.
+// 1024 threads at 64 registers (32 warps per SM), 16 staged pairs per warp.
 constexpr int GRAD_THREADS = 1024, GRAD_CHUNK = 16;
-constexpr size_t GRAD_SMEM = (size_t)(GRAD_THREADS / 32) * GRAD_CHUNK * sizeof(StageGrad);
+constexpr size_t GRAD_STAGE = (size_t)(GRAD_THREADS / 32) * GRAD_CHUNK * sizeof(StageGrad);
+
+// Floats of a row in shared memory: dL/dtau per pixel, and per tile node the sum
+// over the tile's pixels of the node's interpolation weight times dL/dtau.
+__host__ __device__ inline size_t grad_row_bytes(int nbins)
+{
+    return sizeof(float) * ((size_t)nbins + (size_t)TILE_M * (nbins / TILE_W));
+}
+
+// The far wing of the three sums at V: polynomials in 1/V^2 (Tau32::inner's A,
+// unscaled; sum w dH/du = -d/dV of the first).
+__device__ __forceinline__ GradSums grad_far(const StageGrad &g, float V)
+{
+    const float iv = __fdividef(1.0f, V), W = iv * iv;
+    float d = g.s.A[MP_R - 1], v = (float)(2 * MP_R) * d, t = g.D[MP_R - 1];
+#pragma unroll
+    for (int r = MP_R - 2; r >= 0; r--) {
+        const float A = g.s.A[r];
+        d = fmaf(d, W, A);
+        v = fmaf(v, W, (float)(2 * r + 2) * A);
+        t = fmaf(t, W, g.D[r]);
+    }
+    return {d * W, v * W * iv, t * W};
+}
 
 // One warp, one FP32-walk pair: dL/d(dens), dL/d(v_los), dL/dT summed over the
-// pair's window (all lanes hold the sums afterwards).
-__device__ __forceinline__ void grad_pair32(const Tau32 &s, const double *gt, int nbins,
-                                            float tautail, int lane, const float2 *vtab,
-                                            float &ad, float &av, float &at)
+// pair's window (every lane holds its part afterwards).  The walk is the
+// forward's: pixel steps, and where the forward deposits through the nodes of
+// far-field tiles, the transpose of that, the pair's value at each node times
+// the node's share of dL/dtau (grow: the row's pixels, gnode: its nodes; gnode
+// null: every pixel).  128^3, 1024 sightlines x 1115 pixels: 8.66 ms with all
+// seven nodes at every pixel of the window, 5.2 ms so.
+__device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, const float *grow,
+                                            const float *gnode, int nbins, float tautail,
+                                            int lane, const float2 *vtab, float &ad, float &av,
+                                            float &at)
 {
     const int half = nbins / 2;
     const int j0 = s.j0;
     const float lane_f = (float)lane;
+    const float dmin = fmaxf(s.vmp, TILE_DIST * s.vk);
+    float vsure = -1.f;
     ad = av = at = 0.f;
     for (int dir = 0; dir < 2; dir++) {
-        float kf = dir == 0 ? lane_f : -1.0f - lane_f;
-        const float dkf = dir == 0 ? 32.0f : -32.0f;
-        for (int step = 0; step < half; step += 32, kf += dkf) {
-            const int k = step + lane;
-            const bool valid = k < half;
-            const int koff = dir == 0 ? k : -1 - k;
-            const float vlow_b = fmaf(kf, s.bintov, s.base0) * s.inv_b;
-            GradSums g;
-            if (s.npoints == 1) {
-                g = grad_node_sums(s, vlow_b + s.hbin_b, vtab);
-            } else {
-                g = grad_node_sums(s, vlow_b, vtab);
-                g.d *= 0.5f;
-                g.v *= 0.5f;
-                g.t *= 0.5f;
-                for (int i = 1; i < s.npoints - 1; ++i) {
-                    const GradSums h = grad_node_sums(s, fmaf((float)i, s.sub_dv, vlow_b), vtab);
-                    g.d += h.d;
-                    g.v += h.v;
-                    g.t += h.t;
+        bool far = false, tiles = s.tiles && gnode != nullptr;
+        int k = 0, n = 0, items = 0, base = 0, jb_run = 0;
+        while (k < half) {
+            const int koff0 = dir == 0 ? k : -1 - k;
+            const float kf0 = (float)koff0;
+            int len = 32;
+            if (items == 0 && tiles) {
+                if (!far) {
+                    const float ve = dir == 0 ? fmaf(kf0, s.vk, s.v0) : -fmaf(kf0 + 1.f, s.vk, s.v0);
+                    far = ve >= dmin;
                 }
-                const GradSums h = grad_node_sums(s, vlow_b + 2.f * s.hbin_b, vtab);
-                g.d += 0.5f * h.d;
-                g.v += 0.5f * h.v;
-                g.t += 0.5f * h.t;
+                if (far) {
+                    const int jb = bin_from(j0, koff0, nbins);
+                    const int rem = dir == 0 ? (TILE_W - jb % TILE_W) % TILE_W
+                                             : (jb + 1) % TILE_W;
+                    if (rem == 0) {
+                        if (vsure < 0.f)
+                            vsure = 0.999f * far_stop_radius(s, tautail);
+                        const float klim = dir == 0 ? (vsure - s.vmid0) / s.vk
+                                                    : (vsure + s.vmid0) / s.vk - 1.f;
+                        n = 0;
+                        if (klim >= (float)k + (float)(TILE_W - 1))
+                            n = (int)fminf((klim - (float)k + 1.f) / (float)TILE_W, 1e6f);
+                        n = min(n, (half - k) / TILE_W);
+                        n = min(n, dir == 0 ? (nbins - jb) / TILE_W : (jb + 1) / TILE_W);
+                        if (n > 0) {
+                            items = n * TILE_M;
+                            base = 0;
+                            jb_run = jb;
+                        } else {
+                            tiles = dir == 0 ? (nbins - jb < TILE_W) : false;
+                        }
+                    } else {
+                        len = min(32, rem);
+                    }
+                }
             }
-            const float tl = s.scale * g.d;
-            const unsigned m = __ballot_sync(0xffffffffu, valid && tl < tautail);
-            const int last = m ? (__ffs(m) - 1) : 31;
-            if (valid && lane <= last) {
-                const float gg = (float)gt[bin_from(j0, koff, nbins)];
-                ad = fmaf(gg, g.d, ad);
-                av = fmaf(gg, g.v, av);
-                at = fmaf(gg, g.t, at);
+            // one evaluation per lane: a tile node or a pixel, and its dL/dtau
+            float x, gg = 0.f;
+            bool on;
+            if (items) {
+                const int it0 = base + lane;
+                on = it0 < items;
+                const int it = on ? it0 : 0;
+                const int t = it / TILE_M, m = it - t * TILE_M;
+                const int kt = k + TILE_W * t;
+                x = fmaf((float)(dir == 0 ? kt : -kt - TILE_W), s.vk, s.v0);
+                x = fmaf(g_tile.x[m], s.vk, x);
+                if (on)
+                    gg = gnode[(dir == 0 ? jb_run + TILE_W * t
+                                         : jb_run - TILE_W * (t + 1) + 1) / TILE_W * TILE_M + m];
+            } else {
+                const int kk = k + lane;
+                on = lane < len && kk < half;
+                x = fmaf(dir == 0 ? kf0 + lane_f : kf0 - lane_f, s.bintov, s.base0) * s.inv_b;
+                if (on)
+                    gg = grow[bin_from(j0, dir == 0 ? kk : -1 - kk, nbins)];
             }
-            if (m)
+            GradSums r = {0.f, 0.f, 0.f};
+            const int np = s.npoints;
+            for (int i = 0; i < np; i++) {
+                const float xi = np == 1 ? x + s.hbin_b
+                                         : (i == np - 1 ? x + 2.f * s.hbin_b
+                                                        : fmaf((float)i, s.sub_dv, x));
+                const GradSums h = __all_sync(0xffffffffu, fabsf(xi) >= s.vmp)
+                                       ? grad_far(g, xi) : grad_node_sums(s, xi, vtab);
+                const float wt = np > 1 && (i == 0 || i == np - 1) ? 0.5f : 1.f;
+                r.d = fmaf(wt, h.d, r.d);
+                r.v = fmaf(wt, h.v, r.v);
+                r.t = fmaf(wt, h.t, r.t);
+            }
+            unsigned msk = 0;
+            if (!items) {
+                msk = __ballot_sync(0xffffffffu, on && s.scale * r.d < tautail);
+                on = on && lane <= (msk ? __ffs(msk) - 1 : 31);
+            }
+            if (on) {
+                ad = fmaf(gg, r.d, ad);
+                av = fmaf(gg, r.v, av);
+                at = fmaf(gg, r.t, at);
+            }
+            if (items) {
+                base += 32;
+                if (base >= items) {
+                    k += TILE_W * n;
+                    items = 0;
+                }
+                continue;
+            }
+            if (msk)
                 break;
+            k += len;
         }
     }
 }
 
-// Sightlines from a ticket queue; within a sightline the warps take chunks of
-// pairs from a shared counter, each lane sets up one pair of the chunk (the
-// forward's lane-parallel setup) and the warp walks them one after another.
+// Sightlines from a ticket queue; per sightline the row of dL/dtau goes to shared
+// memory as floats with its projection on the tile nodes, then the warps take
+// chunks of pairs from a shared counter, each lane sets up one pair of the chunk
+// (the forward's lane-parallel setup) and the warp walks them one after another.
 __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
 {
     extern __shared__ __align__(16) unsigned char gsmem[];
@@ -2694,6 +2792,11 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
     const float bintov_f = (float)bintov_d;
     const Setup32 k32(a.lp, bintov_d);
     StageGrad *sw = reinterpret_cast<StageGrad *>(gsmem) + warp * GRAD_CHUNK;
+    // the row of dL/dtau (in global memory when it is too long)
+    float *grow = a.rows ? a.rows + (size_t)blockIdx.x * (grad_row_bytes(nbins) / sizeof(float))
+                         : reinterpret_cast<float *>(gsmem + GRAD_STAGE);
+    float *gnode = grow + nbins;
+    const int nnodes = TILE_M * (nbins / TILE_W);
     if (threadIdx.x == 0)
         s_ticket = atomicAdd(a.ticket, 1u);
     __syncthreads();
@@ -2703,8 +2806,18 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
         const int axis = a.t.axis[line];
         const double *gt = a.grad_tau + (size_t)line * nbins;
         const long long e0 = a.pl.off[line], e1 = a.pl.off[line + 1];
+        for (int j = threadIdx.x; j < nbins; j += blockDim.x)
+            grow[j] = (float)gt[j];
         if (threadIdx.x == 0)
             s_chunk = 0u;
+        for (int j = threadIdx.x; j < nnodes; j += blockDim.x) {
+            const double *row = gt + j / TILE_M * TILE_W;
+            const double *w = g_tile.w + j % TILE_M;
+            double sum = 0.0;
+            for (int p = 0; p < TILE_W; p++)
+                sum = fma(w[p * TILE_M], row[p], sum);
+            gnode[j] = (float)sum;
+        }
         __syncthreads();
         for (;;) {
             unsigned c = 0;
@@ -2721,13 +2834,13 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
                 g.temp = in.temp;
                 g.ip = a.pl.part[cb + lane];
                 g.pad = 0;
-                if (!stage32_setup(a.lp, k32, in, bintov_d, g.s, &g.scale_nod))
+                if (!stage32_setup(a.lp, k32, in, bintov_d, g.s, &g.scale_nod, g.D))
                     g.s.flags = STAGE_SKIP;
                 sw[lane] = g;
             }
             __syncwarp();
             for (int k = 0; k < n; k++) {
-                const StageGrad g = sw[k];
+                const StageGrad &g = sw[k];
                 if (g.s.flags & STAGE_SKIP)
                     continue;
                 float gd = 0.f, gv = 0.f, gtmp = 0.f;
@@ -2742,7 +2855,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
                     Tau32 s;
                     s.load(g.s, bintov_f);
                     float ad, av, at;
-                    grad_pair32(s, gt, nbins, tautail, lane, vtab, ad, av, at);
+                    grad_pair32(g, s, grow, gnode, nbins, tautail, lane, vtab, ad, av, at);
                     gd = g.scale_nod * ad;
                     gv = s.scale * s.inv_b * av;
                     gtmp = -s.scale / (2.0f * g.temp) * at;
@@ -2775,7 +2888,8 @@ int g_max_smem_optin = -1;
 // 768- and 1024-thread builds beside the default.
 // The kernel build for a block size and input path: the FP32 optical-depth
 // deposit has 512-, 768- and 1024-thread builds, each gathering the particle
-// fields or reading pair records.
+// fields or reading pair records; the FP32 column density has 512- and
+// 1024-thread builds (104 and 64 registers; the tuner's choice).
 template <bool TAU, int PREC, bool COUNT>
 decltype(&deposit_kernel<TAU, PREC, COUNT>) deposit_build(int threads, bool rec)
 {
@@ -2791,6 +2905,10 @@ decltype(&deposit_kernel<TAU, PREC, COUNT>) deposit_build(int threads, bool rec)
             return deposit_kernel<TAU, PREC, COUNT, 1024, false>;
         if (threads > 512)
             return deposit_kernel<TAU, PREC, COUNT, 768, false>;
+    }
+    if constexpr (!TAU && PREC == 1 && !COUNT) {
+        if (threads > 512)
+            return deposit_kernel<TAU, PREC, COUNT, 1024, false>;
     }
     (void)rec;
     return deposit_kernel<TAU, PREC, COUNT>;
@@ -3046,10 +3164,6 @@ int launch_deposit(const LineParams &lp, const LineTables &t, const Particles &p
         k<<<cfg.persistent ? cfg.grid : nlos, cfg.threads, smem, s>>>(a);
         return launched;
     }
-    if (cfg.tiles && counters == nullptr) {
-        tile_weights_kernel<<<1, TILE_W * TILE_M, 0, s>>>();
-        launched++;
-    }
     const int grid = cfg.persistent ? cfg.grid : nlos;
     const int threads = cfg.threads;
     const bool count = counters != nullptr;
@@ -3102,7 +3216,8 @@ void launch_deposit_fallback_dev(const LineParams &lp, const LineTables &t, cons
 void launch_tau_backward(const LineParams &lp, const LineTables &t, const Particles &p,
                          const PairLists &pl, const int *line_order, int nlos,
                          const double *grad_tau, float *g_dens, float *g_temp, float *g_vel,
-                         unsigned *ticket, unsigned *dev_err, int grid, cudaStream_t s)
+                         unsigned *ticket, unsigned *dev_err, float *rows, int grid,
+                         cudaStream_t s)
 {
     if (nlos == 0 || lp.nbins == 0)
         return;
@@ -3119,17 +3234,24 @@ void launch_tau_backward(const LineParams &lp, const LineTables &t, const Partic
     a.g_vel = g_vel;
     a.ticket = ticket;
     a.dev_err = dev_err;
-    cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)GRAD_SMEM);
-    grad_kernel<<<grid, GRAD_THREADS, GRAD_SMEM, s>>>(a);
+    a.rows = rows;
+    const size_t smem = GRAD_STAGE + (rows ? 0 : grad_row_bytes(lp.nbins));
+    cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    grad_kernel<<<grid, GRAD_THREADS, smem, s>>>(a);
 }
 
-int tau_backward_resident_ctas()
+size_t tau_backward_row_bytes(int nbins)
+{
+    const size_t row = grad_row_bytes(nbins);
+    return GRAD_STAGE + row <= (size_t)(max_smem_optin() - STATIC_SMEM_RESERVE) ? 0 : row;
+}
+
+int tau_backward_resident_ctas(int nbins)
 {
     int n = 0;
-    cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)GRAD_SMEM);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grad_kernel, GRAD_THREADS, GRAD_SMEM);
+    const size_t smem = GRAD_STAGE + (tau_backward_row_bytes(nbins) ? 0 : grad_row_bytes(nbins));
+    cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grad_kernel, GRAD_THREADS, smem);
     return n;
 }
 

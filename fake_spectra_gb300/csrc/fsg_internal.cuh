@@ -334,8 +334,12 @@ int deposit_max_smem_bins(int compute_tau, int precision, int threads);
 void launch_tau_backward(const LineParams &lp, const LineTables &t, const Particles &p,
                          const PairLists &pl, const int *line_order, int nlos,
                          const double *grad_tau, float *g_dens, float *g_temp, float *g_vel,
-                         unsigned *ticket, unsigned *dev_err, int grid, cudaStream_t s);
-int tau_backward_resident_ctas();
+                         unsigned *ticket, unsigned *dev_err, float *rows, int grid,
+                         cudaStream_t s);
+int tau_backward_resident_ctas(int nbins);
+// Device memory per block for rows too long for shared memory (then `rows` is
+// grid times this; else 0 and null).
+size_t tau_backward_row_bytes(int nbins);
 
 // Peak FMA throughput of this GPU (TFLOP/s, 2 flops per FMA), own microbenchmark.
 double measure_fma_peak(int precision, cudaStream_t s);
