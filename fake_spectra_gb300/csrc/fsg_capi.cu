@@ -10,6 +10,7 @@
 //      sightlines with non-finite contributions re-run by the fallback kernel.
 #include "fsg.h"
 
+#include "fsg_fexp.cuh"
 #include "fsg_internal.cuh"
 
 #include <algorithm>
@@ -428,11 +429,11 @@ long long near_lines(fsg_context *c, const Particles &p, int *out)
 }
 
 // The table of the flux passes' exponential on the device (uploaded once).
-const double *exp_table(fsg_context *c)
+const uint64_t *exp_table(fsg_context *c)
 {
-    auto *t = (double *)c->ensure(c->fexp, sizeof(double) * 256);
+    auto *t = (uint64_t *)c->ensure(c->fexp, sizeof(uint64_t) * EXP_TABLE);
     if (!c->fexp_ready) {
-        double h[256];
+        uint64_t h[EXP_TABLE];
         exp_table_host(h);
         cuda_check(cudaMemcpyAsync(t, h, sizeof h, cudaMemcpyHostToDevice, c->stream), "H2D");
         cuda_check(cudaStreamSynchronize(c->stream), "exp table");
@@ -452,7 +453,7 @@ double mean_flux_scale(fsg_context *c, const double *tau, long long n, double mf
                        double thresh)
 {
     cudaStream_t s = c->stream;
-    const double *etab = exp_table(c);
+    const uint64_t *etab = exp_table(c);
     auto *part = (double *)c->ensure(c->fpart, sizeof(double) * flux_partials(3));
     auto *state = (double *)c->ensure(c->fout, sizeof(double) * 4);
     const double init[4] = {1.0, 1.0, 0.0, 0.0};
@@ -481,7 +482,7 @@ double mean_flux_scale(fsg_context *c, const double *tau, long long n, double mf
 double mean_flux_of(fsg_context *c, const double *tau, long long n, double scale)
 {
     cudaStream_t s = c->stream;
-    const double *etab = exp_table(c);
+    const uint64_t *etab = exp_table(c);
     auto *part = (double *)c->ensure(c->fpart, sizeof(double) * flux_partials(3));
     auto *out = (double *)c->ensure(c->fout, sizeof(double) * 4);
     cuda_check(cudaEventRecord(c->ev[2], s), "event");
@@ -1910,7 +1911,7 @@ int fsg_flux_exp_device(fsg_context *ctx, const double *y, int64_t n, double *ou
         if (n < 0)
             fail(FSG_ERR_VALUE, "n must be >= 0 (got %lld)", (long long)n);
         cuda_check(cudaSetDevice(ctx->device), "cudaSetDevice");
-        const double *etab = exp_table(ctx);
+        const uint64_t *etab = exp_table(ctx);
         if (n > 0) {
             launch_fexp(y, n, etab, out, ctx->stream);
             ctx->stats.gpu_launches++;
@@ -1994,7 +1995,7 @@ int fsg_flux_power_device(fsg_context *ctx, const double *tau, int64_t nspec, in
             cuda_check(cudaStreamSynchronize(s), "flux power tables");
             pl = fresh;
         }
-        const double *etab = exp_table(ctx);
+        const uint64_t *etab = exp_table(ctx);
         const long long chunk = power_pairs_per_chunk(pl, nspec);
         const size_t words = sizeof(double2) * (size_t)chunk * (size_t)pl.len;
         auto *a = (double2 *)ctx->ensure(ctx->fdflux, words);

@@ -44,6 +44,15 @@ __device__ __forceinline__ void block_range(long long n, long long &lo, long lon
     hi = lo + per < n ? lo + per : n;
 }
 
+// The exponential's table in shared memory (the lanes of a warp read 32 different
+// entries).
+__device__ __forceinline__ void load_exp_table(uint64_t *tab, const uint64_t *etab)
+{
+    for (int k = threadIdx.x; k < EXP_TABLE; k += blockDim.x)
+        tab[k] = etab[k];
+    __syncthreads();
+}
+
 // Newton-Raphson on the device (py_module.cpp:242-258): state[0] = the scale
 // of the last pass, state[1] = the next scale, state[2] = 1 once converged,
 // state[3] = passes.  A pass reads the scale from state[1]; once state[2] is
@@ -51,12 +60,15 @@ __device__ __forceinline__ void block_range(long long n, long long &lo, long lon
 // iterations between reads.
 __global__ void __launch_bounds__(RED_THREADS)
     flux_moments_dev_kernel(const double *tau, long long n, const double *state, double thresh,
-                            const double *etab, double *part)
+                            const uint64_t *etab, double *part)
 {
     __shared__ double scratch[RED_THREADS / 32];
+    __shared__ uint64_t tab[EXP_TABLE];
     if (state[2] != 0.0)
         return;
-    const double scale = state[1];
+    const double nscale = -state[1];
+    const ExpScale es = exp_scale(nscale);
+    load_exp_table(tab, etab);
     long long lo, hi;
     block_range(n, lo, hi);
     double f = 0.0, tf = 0.0;
@@ -66,7 +78,6 @@ __global__ void __launch_bounds__(RED_THREADS)
     // false as in FP64), else in FP64
     const long long thr_bits = __double_as_longlong(thresh);
     const bool int_cmp = thr_bits >= 0;
-    const double nscale = -scale;
     for (long long i = lo + threadIdx.x; i < hi; i += RED_THREADS) {
         const double t = tau[i];
         const long long tb = __double_as_longlong(t);
@@ -75,7 +86,7 @@ __global__ void __launch_bounds__(RED_THREADS)
                                    : t > thresh;
         if (above)
             continue;
-        const double e = fexp(nscale * t, etab);
+        const double e = fexp(t, nscale, es, tab);
         f += e;
         tf = fma(e, t, tf);
         cnt++;
@@ -129,15 +140,18 @@ __global__ void newton_update_kernel(const double *part, int nblocks, double mfd
 
 // Sum of exp(-scale tau) over all pixels (np.mean(np.exp(-tau)) with scale 1).
 __global__ void __launch_bounds__(RED_THREADS) flux_sum_kernel(const double *tau, long long n,
-                                                               double scale, const double *etab,
+                                                               double scale, const uint64_t *etab,
                                                                double *part)
 {
     __shared__ double scratch[RED_THREADS / 32];
+    __shared__ uint64_t tab[EXP_TABLE];
+    const ExpScale es = exp_scale(-scale);
+    load_exp_table(tab, etab);
     long long lo, hi;
     block_range(n, lo, hi);
     double f = 0.0;
     for (long long i = lo + threadIdx.x; i < hi; i += RED_THREADS)
-        f += fexp(-scale * tau[i], etab);
+        f += fexp(tau[i], -scale, es, tab);
     f = block_sum_ordered(f, scratch);
     if (threadIdx.x == 0)
         part[blockIdx.x] = f;
@@ -330,7 +344,7 @@ __global__ void __launch_bounds__(FLUX_HIST_THREADS)
 }  // namespace
 
 void launch_newton_passes(const double *tau, long long n, double mfd, double tol, double thresh,
-                          int passes, const double *etab, double *part, double *state,
+                          int passes, const uint64_t *etab, double *part, double *state,
                           cudaStream_t s)
 {
     for (int k = 0; k < passes; k++) {
@@ -340,7 +354,7 @@ void launch_newton_passes(const double *tau, long long n, double mfd, double tol
     }
 }
 
-void launch_flux_sum(const double *tau, long long n, double scale, const double *etab,
+void launch_flux_sum(const double *tau, long long n, double scale, const uint64_t *etab,
                      double *part, double *out1, cudaStream_t s)
 {
     flux_sum_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(tau, n, scale, etab, part);
@@ -348,25 +362,26 @@ void launch_flux_sum(const double *tau, long long n, double scale, const double 
 }
 
 // out[i] = exp(y[i]) as the flux passes evaluate it
-__global__ void fexp_kernel(const double *y, long long n, const double *etab, double *out)
+__global__ void fexp_kernel(const double *y, long long n, const uint64_t *etab, double *out)
 {
+    const ExpScale one = exp_scale(1.0);
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        out[i] = fexp(y[i], etab);
+        out[i] = fexp(y[i], 1.0, one, etab);
 }
 
-void launch_fexp(const double *y, long long n, const double *etab, double *out, cudaStream_t s)
+void launch_fexp(const double *y, long long n, const uint64_t *etab, double *out, cudaStream_t s)
 {
     long long blocks = (n + 255) / 256;
     blocks = blocks < 1 ? 1 : (blocks > 4096 ? 4096 : blocks);
     fexp_kernel<<<(unsigned)blocks, 256, 0, s>>>(y, n, etab, out);
 }
 
-void exp_table_host(double *tab)
+void exp_table_host(uint64_t *tab)
 {
-    // 2^(j/256) in extended precision, rounded once to double
-    for (int j = 0; j < 256; j++)
-        tab[j] = (double)std::exp2l((long double)j / 256.0L);
+    // 2^(63 - k/1024) in extended precision, rounded once
+    for (int k = 0; k < EXP_TABLE; k++)
+        tab[k] = (uint64_t)(std::exp2l(63.0L - (long double)k / EXP_TABLE) + 0.5L);
 }
 
 size_t flux_partials(int width) { return (size_t)RED_BLOCKS * width; }

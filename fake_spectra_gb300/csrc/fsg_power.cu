@@ -342,18 +342,19 @@ __global__ void chirp_filter_kernel(const double2 *w, unsigned N, unsigned M, do
 __global__ void power_pack_kernel(const double *__restrict__ tau, unsigned rows, unsigned N,
                                   unsigned L, double scale, double inv_mean,
                                   const double2 *__restrict__ chirp,
-                                  const double *__restrict__ etab, double2 *__restrict__ z,
+                                  const uint64_t *__restrict__ etab, double2 *__restrict__ z,
                                   unsigned total)
 {
+    const ExpScale es = exp_scale(-scale);
     const unsigned stride = gridDim.x * blockDim.x;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const unsigned p = i / L, n = i - p * L;
         double2 v = make_double2(0.0, 0.0);
         if (n < N) {
             const size_t ra = 2 * (size_t)p;
-            v.x = fma(fexp(-scale * tau[ra * N + n], etab), inv_mean, -1.0);
+            v.x = fma(fexp(tau[ra * N + n], -scale, es, etab), inv_mean, -1.0);
             if (ra + 1 < rows)
-                v.y = fma(fexp(-scale * tau[(ra + 1) * N + n], etab), inv_mean, -1.0);
+                v.y = fma(fexp(tau[(ra + 1) * N + n], -scale, es, etab), inv_mean, -1.0);
             if (chirp)
                 v = cmul(v, chirp[n]);
         }
@@ -560,7 +561,7 @@ long long power_pairs_per_chunk(const PowerPlan &pl, long long nspec)
 }
 
 int power_chunk(const PowerPlan &pl, const double2 *tables, const double2 *chirp,
-                const double2 *bhat, const double *etab, const double *tau, long long rows,
+                const double2 *bhat, const uint64_t *etab, const double *tau, long long rows,
                 double scale, double inv_mean, double vmax, double2 *a, double2 *b,
                 double *partial, double *power, cudaStream_t s)
 {
