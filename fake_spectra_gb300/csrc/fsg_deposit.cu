@@ -2666,7 +2666,7 @@ __device__ __forceinline__ GradSums grad_far(const StageGrad &g, float V)
 // far-field tiles, the transpose of that, the pair's value at each node times
 // the node's share of dL/dtau (grow: the row's pixels, gnode: its nodes; gnode
 // null: every pixel).  128^3, 1024 sightlines x 1115 pixels: 8.66 ms with all
-// seven nodes at every pixel of the window, 5.2 ms so.
+// seven nodes at every pixel of the window, 5.4 ms so.
 __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, const float *grow,
                                             const float *gnode, int nbins, float tautail,
                                             int lane, const float2 *vtab, float &ad, float &av,
@@ -2694,11 +2694,14 @@ __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, 
                     const int jb = bin_from(j0, koff0, nbins);
                     const int rem = dir == 0 ? (TILE_W - jb % TILE_W) % TILE_W
                                              : (jb + 1) % TILE_W;
-                    if (rem == 0) {
-                        if (vsure < 0.f)
-                            vsure = 0.999f * far_stop_radius(s, tautail);
-                        const float klim = dir == 0 ? (vsure - s.vmid0) / s.vk
-                                                    : (vsure + s.vmid0) / s.vk - 1.f;
+                    if (vsure < 0.f)
+                        vsure = 0.999f * far_stop_radius(s, tautail);
+                    const float klim = dir == 0 ? (vsure - s.vmid0) / s.vk
+                                                : (vsure + s.vmid0) / s.vk - 1.f;
+                    if (!(klim >= (float)(k + rem) + (float)(TILE_W - 1)) ||
+                        half - k - rem < TILE_W) {
+                        tiles = false;     // the window ends before the next tile does
+                    } else if (rem == 0) {
                         n = 0;
                         if (klim >= (float)k + (float)(TILE_W - 1))
                             n = (int)fminf((klim - (float)k + 1.f) / (float)TILE_W, 1e6f);
@@ -2716,8 +2719,9 @@ __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, 
                     }
                 }
             }
-            // one evaluation per lane: a tile node or a pixel, and its dL/dtau
-            float x, gg = 0.f;
+            // one evaluation per lane: a tile node or a pixel, and its dL/dtau; the
+            // position is x mul (mul: to units of b) plus the sample's offset
+            float x, mul = 1.f, gg = 0.f;
             bool on;
             if (items) {
                 const int it0 = base + lane;
@@ -2733,23 +2737,37 @@ __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, 
             } else {
                 const int kk = k + lane;
                 on = lane < len && kk < half;
-                x = fmaf(dir == 0 ? kf0 + lane_f : kf0 - lane_f, s.bintov, s.base0) * s.inv_b;
+                x = fmaf(dir == 0 ? kf0 + lane_f : kf0 - lane_f, s.bintov, s.base0);
+                mul = s.inv_b;
                 if (on)
                     gg = grow[bin_from(j0, dir == 0 ? kk : -1 - kk, nbins)];
             }
-            GradSums r = {0.f, 0.f, 0.f};
+            // The stop rule compares with tautail: where the wing polynomial comes
+            // within 1e-4 of it (its own error is 1e-6) the node sums decide.  A stop
+            // one pixel off moves the temperature gradient of a weak particle, whose
+            // window ends on its Gaussian flank, by 1e-3 of the largest.
+            GradSums r;
             const int np = s.npoints;
-            for (int i = 0; i < np; i++) {
-                const float xi = np == 1 ? x + s.hbin_b
-                                         : (i == np - 1 ? x + 2.f * s.hbin_b
-                                                        : fmaf((float)i, s.sub_dv, x));
-                const GradSums h = __all_sync(0xffffffffu, fabsf(xi) >= s.vmp)
-                                       ? grad_far(g, xi) : grad_node_sums(s, xi, vtab);
-                const float wt = np > 1 && (i == 0 || i == np - 1) ? 0.5f : 1.f;
-                r.d = fmaf(wt, h.d, r.d);
-                r.v = fmaf(wt, h.v, r.v);
-                r.t = fmaf(wt, h.t, r.t);
-            }
+            bool nodes = false;
+            do {
+                bool poly = false;
+                r = {0.f, 0.f, 0.f};
+                for (int i = 0; i < np; i++) {
+                    const float xi = np == 1 ? fmaf(x, mul, s.hbin_b)
+                                     : i == np - 1 ? fmaf(x, mul, 2.f * s.hbin_b)
+                                                   : fmaf((float)i, s.sub_dv, __fmul_rn(x, mul));
+                    const bool wing = !nodes && __all_sync(0xffffffffu, fabsf(xi) >= s.vmp);
+                    const GradSums h = wing ? grad_far(g, xi) : grad_node_sums(s, xi, vtab);
+                    const float wt = np > 1 && (i == 0 || i == np - 1) ? 0.5f : 1.f;
+                    r.d = fmaf(wt, h.d, r.d);
+                    r.v = fmaf(wt, h.v, r.v);
+                    r.t = fmaf(wt, h.t, r.t);
+                    poly |= wing;
+                }
+                nodes = poly && !items &&
+                        __any_sync(0xffffffffu, on && fabsf(fmaf(s.scale, r.d, -tautail)) <=
+                                                          1e-4f * tautail);
+            } while (nodes);
             unsigned msk = 0;
             if (!items) {
                 msk = __ballot_sync(0xffffffffu, on && s.scale * r.d < tautail);
