@@ -93,7 +93,7 @@ struct fsg_context {
     DevBuf skey, sperm, shist, sstart, ssums;                // particle ordering
     DevBuf flag, tcount, tstart, tsums, idx;                 // _near_lines
     DevBuf fpart, fout, fedges, fcounts, ftau, fdflux, ffft, fpower;   // flux statistics
-    DevBuf ptables, pchirp, pbhat, ppart;                    // flux power plan and partials
+    DevBuf ptables, pchirp, pbhat, pfused, ppart;            // flux power plan and partials
     DevBuf fexp;                                             // 2^(j/256) of the flux exponential
     bool fexp_ready = false;
     PowerPlan pplan;                                         // plan of the last flux power call
@@ -182,7 +182,8 @@ struct fsg_context {
                           &line_order, &ticket, &bad, &nbad, &err, &gacc, &counters,
                           &skey, &sperm, &shist, &sstart, &ssums, &flag, &tcount, &tstart,
                           &tsums, &idx, &fpart, &fout, &fedges, &fcounts, &ftau, &fdflux,
-                          &ffft, &fpower, &ptables, &pchirp, &pbhat, &ppart, &fexp, &vseg,
+                          &ffft, &fpower, &ptables, &pchirp, &pbhat, &pfused, &ppart, &fexp,
+                          &vseg,
                           &vscratch, &vcofm, &tune_order, &prec, &split, &gorder};
         pplan = PowerPlan{};
         fexp_ready = false;
@@ -1990,27 +1991,36 @@ int fsg_flux_power_device(fsg_context *ctx, const double *tau, int64_t nspec, in
                 scratch = (double2 *)ctx->ensure(ctx->ffft, sizeof(double2) * (size_t)fresh.len);
             }
             ctx->stats.gpu_launches += power_plan_tables(fresh, tables, chirp, bhat, scratch, s);
+            if (fresh.in_smem)
+                ctx->stats.gpu_launches += power_fused_tables(
+                    fresh, chirp, bhat, ctx->ensure(ctx->pfused, power_fused_bytes(fresh)), s);
             cuda_check(cudaGetLastError(), "flux power tables");
             // the scratch buffer is regrown below
             cuda_check(cudaStreamSynchronize(s), "flux power tables");
             pl = fresh;
         }
         const uint64_t *etab = exp_table(ctx);
-        const long long chunk = power_pairs_per_chunk(pl, nspec);
-        const size_t words = sizeof(double2) * (size_t)chunk * (size_t)pl.len;
-        auto *a = (double2 *)ctx->ensure(ctx->fdflux, words);
-        auto *b = (double2 *)ctx->ensure(ctx->ffft, words);
         auto *part = (double *)ctx->ensure(ctx->ppart, sizeof(double) * power_partials(npix));
         auto *dp = (double *)ctx->ensure(ctx->fpower, sizeof(double) * nk);
         cuda_check(cudaMemsetAsync(dp, 0, sizeof(double) * nk, s), "memset");
         cuda_check(cudaEventRecord(ctx->ev[2], s), "event");
-        for (long long r0 = 0; r0 < nspec; r0 += 2 * chunk) {
-            const long long r = (r0 + 2 * chunk <= nspec) ? 2 * chunk : nspec - r0;
-            ctx->stats.gpu_launches += power_chunk(
-                pl, (const double2 *)ctx->ptables.p, (const double2 *)ctx->pchirp.p,
-                (const double2 *)ctx->pbhat.p, etab, tau + r0 * npix, r, scale, 1.0 / mean_flux,
-                vmax, a, b, part, dp, s);
+        if (pl.in_smem) {
+            ctx->stats.gpu_launches += power_fused(pl, ctx->pfused.p, etab, tau, nspec, scale,
+                                                   1.0 / mean_flux, vmax, part, dp, s);
             cuda_check(cudaGetLastError(), "flux power launch");
+        } else {
+            const long long chunk = power_pairs_per_chunk(pl, nspec);
+            const size_t words = sizeof(double2) * (size_t)chunk * (size_t)pl.len;
+            auto *a = (double2 *)ctx->ensure(ctx->fdflux, words);
+            auto *b = (double2 *)ctx->ensure(ctx->ffft, words);
+            for (long long r0 = 0; r0 < nspec; r0 += 2 * chunk) {
+                const long long r = (r0 + 2 * chunk <= nspec) ? 2 * chunk : nspec - r0;
+                ctx->stats.gpu_launches += power_chunk(
+                    pl, (const double2 *)ctx->ptables.p, (const double2 *)ctx->pchirp.p,
+                    (const double2 *)ctx->pbhat.p, etab, tau + r0 * npix, r, scale, 1.0 / mean_flux,
+                    vmax, a, b, part, dp, s);
+                cuda_check(cudaGetLastError(), "flux power launch");
+            }
         }
         cuda_check(cudaEventRecord(ctx->ev[3], s), "event");
         cuda_check(cudaMemcpyAsync(power, dp, sizeof(double) * nk, cudaMemcpyDeviceToHost, s),

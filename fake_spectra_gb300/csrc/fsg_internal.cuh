@@ -239,12 +239,23 @@ struct PowerPass {
     long long tw_off = 0;    // table offset of exp(-2 pi i k r / (ns R)), k < ns, r < R
     long long cs_off = -1;   // odd radix: table offset of (cos, sin)(2 pi t / R), t < R
 };
+// A pass of the transforms in shared memory (fsg_dft_fix.cuh).
+constexpr int FUSED_PASSES = 14;
+struct FusedPass {
+    int radix = 0;
+    unsigned m = 0;           // distance of the butterfly's points
+    unsigned tw = 0;          // table offset
+    int e_dif = 0, e_dit = 0;  // divisions by 2 on the way there and back
+};
 struct PowerPlan {
     long long npix = -1;     // N
     long long len = 0;       // transform length: N, or Bluestein's M >= 2N - 1
     bool bluestein = false;
     std::vector<PowerPass> passes;
     long long table_len = 0;  // double2 entries of the pass tables
+    bool in_smem = false;     // rows fit in shared memory: fixed-point transforms
+    std::vector<FusedPass> fused;
+    double filter_max = 1.0;  // Bluestein: largest modulus of the filter
 };
 PowerPlan power_plan(long long npix);
 // Fills the pass tables (table_len entries) and, for Bluestein, the chirp
@@ -262,6 +273,14 @@ int power_chunk(const PowerPlan &pl, const double2 *tables, const double2 *chirp
                 double scale, double inv_mean, double vmax, double2 *a, double2 *b,
                 double *partial, double *power, cudaStream_t s);
 size_t power_partials(long long npix);
+// pl.in_smem: the tables (power_fused_bytes; from the chirp and bhat for Bluestein)
+// and the power of `rows` sightlines in one launch, as power_chunk.
+size_t power_fused_bytes(const PowerPlan &pl);
+int power_fused_tables(PowerPlan &pl, const double2 *chirp, const double2 *bhat, void *tables,
+                       cudaStream_t s);
+int power_fused(const PowerPlan &pl, const void *tables, const uint64_t *etab, const double *tau,
+                long long rows, double scale, double inv_mean, double vmax, double *partial,
+                double *power, cudaStream_t s);
 
 // After emit: every sightline's cursor must equal its count (DEVERR_PAIR_COUNT
 // otherwise), so no slot of the pair lists is left unwritten.

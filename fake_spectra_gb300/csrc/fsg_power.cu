@@ -1,5 +1,6 @@
 // 1-D flux power spectrum (fake_spectra/fluxstatistics.py:53-110) with the
-// project's own FP64 discrete Fourier transforms.
+// project's own discrete Fourier transforms: in shared memory and 64-bit fixed
+// point for lengths that fit, else FP64 passes over global memory.
 //
 // The reference takes np.fft.rfft of d_F = exp(-s tau) / <F> - 1 along each
 // sightline and sums |rfft|^2 / npix^2 over sightlines.  Here two sightlines a
@@ -21,13 +22,14 @@
 // convolution as conj(FFT(conj(FFT(a) FFT(b)))) / M; |w_k| = 1, so the power is
 // |FFT(conj(FFT(a) FFT(b)))_k|^2 / M^2.
 //
-// GB300 runs FP64 at 1/64 of the FP32 rate, and the transform is FP64-bound
+// GB300 runs FP64 at 1/64 of the FP32 rate, and the FP64 passes are bound by it
 // (the reference's test tolerance of 1e-10 relative leaves no room for FP32
-// arithmetic): the passes keep every table (twiddles, cos/sin of the odd
-// radices) precomputed, and the odd-radix DFT costs about R FMAs per point.
-// Memory traffic (one read and one write of 16 bytes per point and pass) is
-// secondary.  Sums over sightlines go in a fixed order: fixed segments of
-// pairs, each summed in order, then the segments in order.
+// arithmetic): they keep every table (twiddles, cos/sin of the odd radices)
+// precomputed, and the odd-radix DFT costs about R FMAs per point.  They serve
+// rows too long for shared memory (and, once per length, the chirp filter).  Sums
+// over sightlines go in a fixed order: fixed segments of pairs, each summed in
+// order, then the segments in order.
+#include "fsg_dft_fix.cuh"
 #include "fsg_fexp.cuh"
 #include "fsg_internal.cuh"
 
@@ -395,16 +397,255 @@ __global__ void power_partial_kernel(const double2 *__restrict__ Z, unsigned pai
 }
 
 // power[k] += factor * sum over segments (in order) of partial[s][k]
-__global__ void power_combine_kernel(const double *partial, unsigned nk, double factor,
-                                     double *power)
+__global__ void power_combine_kernel(const double *partial, unsigned nk, int segments,
+                                     double factor, double *power)
 {
     const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nk)
         return;
     double sum = 0.0;
-    for (int s = 0; s < POWER_SEGMENTS; s++)
+    for (int s = 0; s < segments; s++)
         sum += partial[(size_t)s * nk + k];
     power[k] += factor * sum;
+}
+
+// ------------------------------------------------- transforms in shared memory
+// Lengths up to FUSED_MAX: a block keeps `batch` sightline pairs in shared memory
+// from the optical depth to |Z_k|^2, in the fixed-point arithmetic of
+// fsg_dft_fix.cuh; global memory holds tau, the tables and one partial sum per
+// block.  Bluestein's two transforms meet in the digit-reversed order the first
+// leaves, so neither reorders, and the last pass of the one, the filter and the
+// first pass of the other run on the same R points in registers.
+//
+// 3600 sightlines x 6691 pixels (length 13440, 10 passes of 16 bytes per point
+// read and written in global memory and about 116 FP64 operations per point):
+// 6.6 ms with the FP64 passes and exponential below, 1.9 ms so.
+constexpr int FUSED_THREADS = 512;
+constexpr int FUSED_BLOCKS = 152;    // fixed: the summation order does not depend on the GPU
+constexpr int FUSED_BATCH = 64;
+constexpr size_t FUSED_SMEM = 227 * 1024 - 2048;   // dynamic; the rest holds the row sums
+constexpr int FUSED_MAX = (int)((FUSED_SMEM - sizeof(uint64_t) * EXP_TABLE) / sizeof(FixC));
+
+struct FusedArgs {
+    const double *tau;
+    long long rows;
+    unsigned N, L;
+    int npass, batch;
+    FusedPass pass[FUSED_PASSES];
+    const FixW *tw, *chirp, *filter;   // chirp, filter: null for a direct transform
+    const unsigned *pos;               // direct: position of frequency k
+    const uint64_t *etab;
+    double scale, inv_mean;
+    int shift;                         // divisions by 2 of all passes
+    double *partial;
+};
+
+enum { PASS_DIF, PASS_DIT, PASS_FILTER };
+
+template <int R, int KIND>
+__device__ __forceinline__ void fused_butterflies(FixC *x, const FixW *tab, unsigned total,
+                                                  unsigned m, unsigned L, int e)
+{
+    for (unsigned f = threadIdx.x; f < total / R; f += FUSED_THREADS) {
+        if constexpr (KIND == PASS_DIF)
+            dif_butterfly<R>(x, tab, f, m, e);
+        else if constexpr (KIND == PASS_DIT)
+            dit_butterfly<R>(x, tab, f, m, e);
+        else
+            filter_butterfly<R>(x, tab, f, L, e);
+    }
+    __syncthreads();
+}
+
+template <int KIND>
+__device__ __forceinline__ void fused_pass(FixC *x, const FixW *tab, unsigned total, int R,
+                                           unsigned m, unsigned L, int e)
+{
+    switch (R) {
+    case 2: fused_butterflies<2, KIND>(x, tab, total, m, L, e); break;
+    case 3: fused_butterflies<3, KIND>(x, tab, total, m, L, e); break;
+    case 4: fused_butterflies<4, KIND>(x, tab, total, m, L, e); break;
+    case 5: fused_butterflies<5, KIND>(x, tab, total, m, L, e); break;
+    case 7: fused_butterflies<7, KIND>(x, tab, total, m, L, e); break;
+    case 8: fused_butterflies<8, KIND>(x, tab, total, m, L, e); break;
+    default: fused_butterflies<16, KIND>(x, tab, total, m, L, e);
+    }
+}
+
+__global__ void __launch_bounds__(FUSED_THREADS, 1) power_fused_kernel(FusedArgs a)
+{
+    extern __shared__ __align__(16) unsigned char fraw[];
+    uint64_t *etab = reinterpret_cast<uint64_t *>(fraw);
+    FixC *x = reinterpret_cast<FixC *>(fraw + sizeof(uint64_t) * EXP_TABLE);
+    __shared__ unsigned long long row_sq[FUSED_BATCH];
+    __shared__ int top;
+    constexpr int NW = FUSED_THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k = threadIdx.x; k < EXP_TABLE; k += FUSED_THREADS)
+        etab[k] = a.etab[k];
+    const ExpScale es = exp_scale(-a.scale);
+    const unsigned N = a.N, L = a.L, nk = N / 2 + 1;
+    const long long pairs = (a.rows + 1) / 2;
+    const long long nbatch = (pairs + a.batch - 1) / a.batch;
+    const long long b0 = nbatch * blockIdx.x / gridDim.x, b1 = nbatch * (blockIdx.x + 1) / gridDim.x;
+    double *partial = a.partial + (size_t)blockIdx.x * nk;
+    for (long long b = b0; b < b1; b++) {
+        const long long p0 = b * a.batch;
+        const int cnt = (int)(pairs - p0 < a.batch ? pairs - p0 : a.batch);
+        if (threadIdx.x < FUSED_BATCH)
+            row_sq[threadIdx.x] = 0ull;
+        if (threadIdx.x == 0)
+            top = 0;
+        __syncthreads();
+        // d = exp(-scale tau) inv_mean - 1 of both sightlines as doubles; a warp
+        // takes one of `parts` stretches of a pair
+        const int parts = (NW + cnt - 1) / cnt;
+        const unsigned len = ((N + parts - 1) / parts + 31) & ~31u;
+        int hmax = 0;
+        for (int u = warp; u < cnt * parts; u += NW) {
+            const int p = u / parts;
+            const unsigned n0 = (u - p * parts) * len, n1 = n0 + len < N ? n0 + len : N;
+            const double *ta = a.tau + 2 * (size_t)(p0 + p) * N;
+            const bool both = 2 * (p0 + p) + 1 < a.rows;
+            double2 *z = reinterpret_cast<double2 *>(x + (size_t)p * L);
+            for (unsigned n = n0 + lane; n < n1; n += 32) {
+                double2 d = make_double2(0.0, 0.0);
+                d.x = fma(fexp(ta[n], -a.scale, es, etab), a.inv_mean, -1.0);
+                if (both)
+                    d.y = fma(fexp(ta[N + n], -a.scale, es, etab), a.inv_mean, -1.0);
+                z[n] = d;
+                hmax = max(hmax, max(__double2hiint(d.x) & 0x7FFFFFFF,
+                                     __double2hiint(d.y) & 0x7FFFFFFF));
+            }
+        }
+        hmax = __reduce_max_sync(0xffffffffu, hmax);
+        if (lane == 0)
+            atomicMax(&top, hmax);
+        __syncthreads();
+        // sums of squares per pair, rounded up, in units of 2^(2 (emax - 21)) of the
+        // largest value's exponent
+        const int hi = top, ehi = hi >> 20, emax = ehi - 1022;
+        for (int u = warp; u < cnt * parts; u += NW) {
+            const int p = u / parts;
+            const unsigned n0 = (u - p * parts) * len, n1 = n0 + len < N ? n0 + len : N;
+            const int2 *z = reinterpret_cast<const int2 *>(x + (size_t)p * L);
+            unsigned long long sq = 0;
+            for (unsigned n = n0 + lane; n < n1; n += 32)
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const int h = z[2 * n + c].y & 0x7FFFFFFF;
+                    const unsigned q = ((((unsigned)h & 0xFFFFFu) | 0x100000u) >>
+                                        min(31, ehi - (h >> 20))) + 1u;
+                    sq += (unsigned long long)q * q;
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            if (lane == 0)
+                atomicAdd(&row_sq[p], sq);
+        }
+        __syncthreads();
+        unsigned long long sq = 1;
+        for (int p = 0; p < cnt; p++)
+            sq = row_sq[p] > sq ? row_sq[p] : sq;
+        // the largest power of two that keeps |z|_2 below 2^60.8 (the bound that the
+        // radix-16 butterflies and fixc_mul allow): 2^121.6 = 1.515 2^121
+        const int l2 = 63 - __clzll((long long)sq);
+        const bool high = ((sq << (63 - l2)) >> 32) > 3253500928ull;   // 1.515 2^31
+        int sh = ((high ? 120 : 121) - l2) / 2 + 21 - emax;
+        if (hi == 0)
+            sh = 0;
+        const bool bad = ehi == 0x7FF;       // an infinity or NaN: every power is NaN
+        // the same in fixed point, times the chirp
+        for (unsigned i = threadIdx.x; i < (unsigned)cnt * L; i += FUSED_THREADS) {
+            const unsigned n = i % L;
+            FixC v = {0, 0};
+            if (n < N && !bad) {
+                const double2 d = reinterpret_cast<const double2 *>(x)[i];
+                if (a.chirp)
+                    v = fixc_mul({fix_from_double(d.x, sh + 2), fix_from_double(d.y, sh + 2)},
+                                 a.chirp[n], 2, 0);
+                else
+                    v = {fix_from_double(d.x, sh), fix_from_double(d.y, sh)};
+            }
+            x[i] = v;
+        }
+        __syncthreads();
+        const unsigned total = (unsigned)cnt * L;
+        const int last = a.npass - 1;
+        for (int i = 0; i < (a.filter ? last : a.npass); i++)
+            fused_pass<PASS_DIF>(x, a.tw + a.pass[i].tw, total, a.pass[i].radix, a.pass[i].m, L,
+                                 a.pass[i].e_dif);
+        if (a.filter) {
+            fused_pass<PASS_FILTER>(x, a.filter, total, a.pass[last].radix, 1, L,
+                                    a.pass[last].e_dif);
+            for (int i = last - 1; i >= 0; i--)
+                fused_pass<PASS_DIT>(x, a.tw + a.pass[i].tw, total, a.pass[i].radix,
+                                     a.pass[i].m, L, a.pass[i].e_dit);
+        }
+        // |Z_k|^2 + |Z_(N-k)|^2; values that square to infinity anyway need no exponent
+        // above 900
+        const int ex = min(a.shift - sh, 900);
+        for (unsigned k = threadIdx.x; k < nk; k += FUSED_THREADS) {
+            const unsigned k2 = k == 0 ? 0 : N - k;
+            const unsigned i1 = a.pos ? a.pos[k] : k, i2 = a.pos ? a.pos[k2] : k2;
+            double sum = b == b0 ? 0.0 : partial[k];
+            for (int p = 0; p < cnt; p++) {
+                const FixC u = x[(size_t)p * L + i1], v = x[(size_t)p * L + i2];
+                const double ux = fix_to_double(u.x, ex), uy = fix_to_double(u.y, ex);
+                const double vx = fix_to_double(v.x, ex), vy = fix_to_double(v.y, ex);
+                sum += fma(ux, ux, uy * uy) + fma(vx, vx, vy * vy);
+            }
+            partial[k] = bad ? __longlong_as_double(0x7FF8000000000000ll) : sum;
+        }
+        __syncthreads();
+    }
+}
+
+// tw[(q - 1) m + j] = exp(-2 pi i j q / (m R))
+__global__ void fused_twiddle_kernel(FixW *tw, unsigned m, int R)
+{
+    const unsigned n = (R - 1) * m;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned q = i / m + 1, j = i - (q - 1) * m;
+        const double2 w = unit_root(-(long long)j * q, (long long)m * R);
+        tw[i] = {fix_v62(w.x), fix_v62(w.y)};
+    }
+}
+
+// largest modulus of b, rounded up (one block)
+__global__ void fused_filter_max_kernel(const double2 *b, unsigned M, double *out)
+{
+    __shared__ unsigned long long top;
+    if (threadIdx.x == 0)
+        top = 0ull;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < M; i += blockDim.x)
+        atomicMax(&top, (unsigned long long)__double_as_longlong(
+                            fma(b[i].x, b[i].x, b[i].y * b[i].y)));
+    __syncthreads();
+    if (threadIdx.x == 0)
+        *out = sqrt(__longlong_as_double((long long)top)) * (1.0 + 1e-14);
+}
+
+// The chirp, and the filter over its largest modulus in the order the first
+// transform leaves.
+__global__ void fused_filter_kernel(FusedArgs a, const double2 *w, const double2 *bhat,
+                                    const double *top, FixW *chirp, FixW *filter)
+{
+    const double inv = 1.0 / *top;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < a.L; i += gridDim.x * blockDim.x) {
+        if (i < a.N)
+            chirp[i] = {fix_v62(w[i].x), fix_v62(w[i].y)};
+        unsigned rest = i, k = 0, mul = 1;
+        for (int p = 0; p < a.npass; p++) {
+            const unsigned d = rest / a.pass[p].m;
+            rest -= d * a.pass[p].m;
+            k += d * mul;
+            mul *= a.pass[p].radix;
+        }
+        filter[i] = {fix_v62(bhat[k].x * inv), fix_v62(bhat[k].y * inv)};
+    }
 }
 
 std::vector<long long> prime_factors(long long n)
@@ -481,16 +722,151 @@ double2 *run_passes(const PowerPlan &pl, const double2 *tables, double2 *x, doub
 
 }  // namespace
 
+namespace {
+
+// Passes of a fused transform of length len (7-smooth): powers of two first (the
+// last pass, over adjacent points, is free of bank conflicts for an odd radix);
+// divisions by 2 so that after combining m points at least sqrt(m) is divided out,
+// 1 or 2 per pass.  Returns an estimate of the instructions per point, 0 when no
+// such plan exists.
+int fused_passes(long long len, bool bluestein, std::vector<FusedPass> &ps)
+{
+    std::vector<int> radix;
+    int twos = 0;
+    for (long long p : prime_factors(len)) {
+        if (p == 2)
+            twos++;
+        else if (p <= 7)
+            radix.push_back((int)p);
+        else
+            return 0;
+    }
+    std::vector<int> order;
+    if (twos % 4 == 1 && twos > 4) {       // 8 x 4 rather than 16 x 2
+        order = {8, 4};
+        twos -= 5;
+    } else if (twos % 4) {
+        order = {1 << twos % 4};
+        twos -= twos % 4;
+    }
+    order.insert(order.begin(), twos / 4, 16);
+    order.insert(order.end(), radix.begin(), radix.end());
+    if (order.size() > FUSED_PASSES)
+        return 0;
+    ps.clear();
+    int cost = 0;
+    unsigned m = (unsigned)len, tw = 0;
+    for (int r : order) {
+        m /= r;
+        FusedPass p;
+        p.radix = r;
+        p.m = m;
+        p.tw = tw;
+        if (m > 1)
+            tw += (r - 1) * m;
+        ps.push_back(p);
+        // instructions per point of the butterfly and its twiddles, and of the
+        // loads, stores and indices
+        cost += 25 + (r == 2 ? 30 : r == 3 ? 53 : r == 4 ? 45 : r == 5 ? 68 : r == 7 ? 100
+                                                              : r == 8 ? 61 : 80);
+    }
+    const auto divisions = [](double half_bits, int done) {
+        const int e = (int)std::ceil(half_bits - 1e-9) - done;
+        return e < 1 ? 1 : e;
+    };
+    double bits = 0.0;
+    int done = 0;
+    for (FusedPass &p : ps) {
+        bits += 0.5 * std::log2((double)p.radix);
+        if (p.m > 1 || bluestein)
+            done += p.e_dif = divisions(bits, done);
+        if (p.e_dif > 2)
+            return 0;
+    }
+    bits = 0.0;
+    done = 0;
+    for (size_t i = ps.size(); bluestein && i-- > 0;) {
+        if (ps[i].m > 1)
+            done += ps[i].e_dit = divisions(bits, done);
+        if (ps[i].e_dit > 2)
+            return 0;
+        bits += 0.5 * std::log2((double)ps[i].radix);
+    }
+    return bluestein ? 2 * cost : cost;
+}
+
+bool smooth7(long long n)
+{
+    for (int p : {2, 3, 5, 7})
+        while (n % p == 0)
+            n /= p;
+    return n == 1;
+}
+
+// The fused plan of npix pixels, if there is one: the length itself when it is
+// 7-smooth, else the cheapest Bluestein length.
+bool fused_plan(long long npix, PowerPlan &pl)
+{
+    pl.bluestein = !smooth7(npix);
+    if (!pl.bluestein) {
+        pl.len = npix;
+        return npix <= FUSED_MAX && (npix == 1 || fused_passes(npix, false, pl.fused) > 0);
+    }
+    long long best = 0;
+    for (long long len = 2 * npix - 1; len <= FUSED_MAX && len < 4 * npix; len++) {
+        std::vector<FusedPass> ps;
+        const int c = smooth7(len) ? fused_passes(len, true, ps) : 0;
+        if (c > 0 && (best == 0 || c * len < best)) {
+            best = c * len;
+            pl.len = len;
+            pl.fused = ps;
+        }
+    }
+    return best > 0;
+}
+
+FusedArgs fused_args(const PowerPlan &pl, const void *tables)
+{
+    FusedArgs a{};
+    a.N = (unsigned)pl.npix;
+    a.L = (unsigned)pl.len;
+    a.npass = (int)pl.fused.size();
+    for (int i = 0; i < a.npass; i++) {
+        a.pass[i] = pl.fused[i];
+        a.shift += a.pass[i].e_dif + a.pass[i].e_dit;
+    }
+    // twiddles, then the chirp and the filter, or the positions
+    a.tw = (const FixW *)tables;
+    const FixW *rest = a.tw + pl.len * (pl.fused.empty() ? 0 : 2);
+    if (pl.bluestein) {
+        a.filter = rest;
+        a.chirp = rest + pl.len;
+    } else {
+        a.pos = (const unsigned *)rest;
+    }
+    return a;
+}
+
+}  // namespace
+
 PowerPlan power_plan(long long npix)
 {
     PowerPlan pl;
     pl.npix = npix;
-    const std::vector<long long> f = prime_factors(npix);
-    long long pmax = 1;
-    for (long long p : f)
-        pmax = p > pmax ? p : pmax;
-    pl.bluestein = pmax > POWER_MAX_ODD_RADIX;
-    pl.len = pl.bluestein ? smooth7_at_least(2 * npix - 1) : npix;
+    pl.in_smem = fused_plan(npix, pl);
+    if (pl.in_smem && !pl.bluestein) {
+        return pl;
+    }
+    if (!pl.in_smem) {
+        pl.fused.clear();
+        const std::vector<long long> f = prime_factors(npix);
+        long long pmax = 1;
+        for (long long p : f)
+            pmax = p > pmax ? p : pmax;
+        pl.bluestein = pmax > POWER_MAX_ODD_RADIX;
+        pl.len = pl.bluestein ? smooth7_at_least(2 * npix - 1) : npix;
+    }
+    // passes of the FP64 transform (fused: of the chirp filter only)
     std::vector<long long> g = prime_factors(pl.len);
     int twos = 0;
     std::vector<int> radix;
@@ -552,6 +928,88 @@ int power_plan_tables(const PowerPlan &pl, double2 *tables, double2 *chirp, doub
     return launches;
 }
 
+size_t power_fused_bytes(const PowerPlan &pl)
+{
+    if (!pl.in_smem)
+        return 0;
+    return sizeof(FixW) * (size_t)pl.len * 4 + sizeof(unsigned) * (size_t)pl.npix + 64;
+}
+
+// Twiddles (fewer than 2 len), chirp and filter or positions; the filter's largest
+// modulus comes back in pl.filter_max (the stream is synchronised).
+int power_fused_tables(PowerPlan &pl, const double2 *chirp, const double2 *bhat, void *tables,
+                       cudaStream_t s)
+{
+    int launches = 0;
+    const FusedArgs a = fused_args(pl, tables);
+    for (const FusedPass &p : pl.fused)
+        if (p.m > 1) {
+            const unsigned n = (p.radix - 1) * p.m;
+            fused_twiddle_kernel<<<grid_for(n, 256), 256, 0, s>>>(
+                const_cast<FixW *>(a.tw) + p.tw, p.m, p.radix);
+            launches++;
+        }
+    pl.filter_max = 1.0;
+    std::vector<unsigned> pos;
+    if (pl.bluestein) {
+        double *top = (double *)const_cast<FixW *>(a.filter + 2 * pl.len);
+        fused_filter_max_kernel<<<1, 1024, 0, s>>>(bhat, a.L, top);
+        fused_filter_kernel<<<grid_for(a.L, 256), 256, 0, s>>>(
+            a, chirp, bhat, top, const_cast<FixW *>(a.chirp), const_cast<FixW *>(a.filter));
+        launches += 2;
+        cudaMemcpyAsync(&pl.filter_max, top, sizeof(double), cudaMemcpyDeviceToHost, s);
+    } else {
+        pos.resize((size_t)pl.npix);
+        for (unsigned i = 0; i < a.N; i++) {
+            unsigned rest = i, k = 0, mul = 1;
+            for (int p = 0; p < a.npass; p++) {
+                const unsigned d = rest / a.pass[p].m;
+                rest -= d * a.pass[p].m;
+                k += d * mul;
+                mul *= a.pass[p].radix;
+            }
+            pos[k] = i;
+        }
+        cudaMemcpyAsync(const_cast<unsigned *>(a.pos), pos.data(), sizeof(unsigned) * pos.size(),
+                        cudaMemcpyHostToDevice, s);
+    }
+    cudaStreamSynchronize(s);
+    return launches;
+}
+
+int power_fused(const PowerPlan &pl, const void *tables, const uint64_t *etab, const double *tau,
+                long long rows, double scale, double inv_mean, double vmax, double *partial,
+                double *power, cudaStream_t s)
+{
+    FusedArgs a = fused_args(pl, tables);
+    a.tau = tau;
+    a.rows = rows;
+    a.etab = etab;
+    a.scale = scale;
+    a.inv_mean = inv_mean;
+    a.partial = partial;
+    // short rows: as many pairs per block as fit, but no fewer blocks than SMs
+    const long long pairs = (rows + 1) / 2;
+    long long batch = std::min<long long>(FUSED_MAX / pl.len, FUSED_BATCH);
+    batch = std::min(batch, (pairs + FUSED_BLOCKS - 1) / FUSED_BLOCKS);
+    a.batch = (int)std::max(1ll, batch);
+    const long long nbatch = (pairs + a.batch - 1) / a.batch;
+    const int blocks = (int)std::min<long long>(nbatch, FUSED_BLOCKS);
+    const size_t smem = sizeof(uint64_t) * EXP_TABLE + sizeof(FixC) * (size_t)a.batch * a.L;
+    cudaFuncSetAttribute(power_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
+    power_fused_kernel<<<blocks, FUSED_THREADS, smem, s>>>(a);
+    double norm = 1.0 / ((double)pl.npix * (double)pl.npix);
+    if (pl.bluestein) {
+        const double g = pl.filter_max / (double)pl.len;
+        norm *= g * g;
+    }
+    const unsigned nk = a.N / 2 + 1;
+    power_combine_kernel<<<(nk + 127) / 128, 128, 0, s>>>(partial, nk, blocks, 0.5 * vmax * norm,
+                                                          power);
+    return 2;
+}
+
 long long power_pairs_per_chunk(const PowerPlan &pl, long long nspec)
 {
     const long long pairs = (nspec + 1) / 2;
@@ -584,12 +1042,15 @@ int power_chunk(const PowerPlan &pl, const double2 *tables, const double2 *chirp
     const unsigned nk = N / 2 + 1;
     power_partial_kernel<<<dim3((nk + 127) / 128, POWER_SEGMENTS), 128, 0, s>>>(r, pairs, L, N,
                                                                               nk, partial);
-    power_combine_kernel<<<(nk + 127) / 128, 128, 0, s>>>(partial, nk, 0.5 * vmax * norm,
-                                                          power);
+    power_combine_kernel<<<(nk + 127) / 128, 128, 0, s>>>(partial, nk, POWER_SEGMENTS,
+                                                          0.5 * vmax * norm, power);
     launches += 2;
     return launches;
 }
 
-size_t power_partials(long long npix) { return (size_t)POWER_SEGMENTS * (npix / 2 + 1); }
+size_t power_partials(long long npix)
+{
+    return (size_t)std::max(POWER_SEGMENTS, FUSED_BLOCKS) * (npix / 2 + 1);
+}
 
 }  // namespace fsg
