@@ -181,6 +181,9 @@ __global__ void partial_sum_kernel(const double *part, int nblocks, int width, d
 // outside the bins, NaN) are decided with the FP64 exponential and numpy's
 // comparisons, so the counts equal numpy's.
 //
+// 2.4e7 pixels, 20 bins: 479 us while the coordinate was rounded to the nearest bin
+// (half of the pixels went to the FP64 recheck), 151 us so.
+//
 // Bins are counted in 32-bit per-warp private histograms in shared memory
 // (nb <= FLUX_WARP_BINS; a warp never counts 2^32 pixels: the grid-stride loop
 // gives each warp at most n / (grid warps) pixels, checked on the host), merged
@@ -273,7 +276,9 @@ __global__ void __launch_bounds__(FLUX_HIST_THREADS)
     __syncthreads();
     const double e0 = edges[0], el = edges[nb];
     const double norm = nb / (el - e0);
-    const float e0f = (float)e0, normf = (float)norm, vmax = (float)(nb - 1);
+    // bin coordinates are clamped inside the last bin: at its lower edge, a tie of the
+    // floor below, every unabsorbed pixel would take the FP64 recheck
+    const float e0f = (float)e0, normf = (float)norm, vmax = (float)(nb - 1) + 0.25f;
     const float sf = trunc_to_float(scale);
     // exp(-scale tau) <= 1 for tau >= 0 and scale >= 0: such a pixel is in the
     // last bin as soon as it clears that bin's lower edge, when the bins reach 1
@@ -295,10 +300,10 @@ __global__ void __launch_bounds__(FLUX_HIST_THREADS)
         // floor of the bin coordinate, clamped, without a float->int conversion
         // (ties at an integer may land one bin low; the test below then fails)
         const float v = fminf(fmaxf((x32 - e0f) * normf, 0.f), vmax);
-        int j = __float_as_int(v + (12582912.0f - 0.5f)) - 0x4B400000;
+        int j = __float_as_int((v - 0.5f) + 12582912.0f) - 0x4B400000;
         j = j < 0 ? 0 : j;
         // certain: [lo, hi] inside [e_j, e_{j+1}) (the last bin: inside [e_j, e_nb])
-        const bool last_ok = j == nb - 1 && (hi <= ed[nb] || (top_closed && t >= 0.0));
+        const bool last_ok = j == nb - 1 && (hi <= ed[nb] || (top_closed && __double2hiint(t) >= 0));
         const bool sure = isfinite(y) && lo >= eu[j] && (hi < ed[j + 1] || last_ok);
         const bool need = valid && !sure;
         hist_add<WARP_PRIVATE>(valid && sure ? j : -1, wh, bh);
