@@ -672,6 +672,9 @@ DepositLaunch deposit_config(fsg_context *c, const LineParams &lp, const fsg_opt
     const bool count = opt && opt->count_work;
     const bool tau32 = cfg.precision == FSG_PREC_FP32 && lp.compute_tau && !vor && !count;
     cfg.rec = tau32 && opt && opt->records == 1;
+    // few sightlines are shared between blocks unless the launch is asked for
+    cfg.split32 = tau32 && !(opt && (opt->threads > 0 || opt->chunk > 0 || opt->persistent >= 0 ||
+                                     opt->records >= 0));
     if (opt && opt->records > 1)
         fail(FSG_ERR_VALUE, "records must be -1 (tuned), 0 or 1");
     cfg.fast64 = cfg.precision == FSG_PREC_FP64 && !count;
@@ -809,7 +812,7 @@ void finish_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
     deposit_fit_chunk(cfg, c->npairs, sms);
     const size_t sb = deposit_split_bytes(cfg, lp.nbins, c->nlos, sms);
     cfg.split_ws = sb ? c->ensure(c->split, sb) : nullptr;
-    cfg.grid = sb ? sms * per_sm : std::min(c->nlos, sms * per_sm);
+    cfg.grid = sb ? sms * (cfg.split32 ? 1 : per_sm) : std::min(c->nlos, sms * per_sm);
 }
 
 // Times the candidate launches on a sample of the call's sightlines (every
@@ -853,6 +856,7 @@ fsg_tune_entry tune_deposit(fsg_context *c, const LineParams &lp, const Particle
     best.sample_lines = nsamp;
     for (const Cand &cd : cands) {
         DepositLaunch cfg = base;
+        cfg.split_ws = nullptr;
         cfg.threads = cd.threads;
         cfg.chunk = cd.chunk;
         cfg.persistent = cd.persistent;

@@ -1784,7 +1784,7 @@ __device__ __forceinline__ void walk_tau32_tiled(const DepositArgs &a, const Tau
 // orders of magnitude); each lane sets up one pair of the chunk into the warp's
 // staging area, then the warp walks the chunk's pairs one after another.
 template <bool COUNT, bool REC>
-__device__ __forceinline__ void deposit_pairs32(const DepositArgs &a, int axis, long long e0,
+__device__ __forceinline__ unsigned deposit_pairs32(const DepositArgs &a, int axis, long long e0,
                                                 long long e1, int S, unsigned long long *lo,
                                                 unsigned long long *hi, unsigned long long *tlo,
                                                 unsigned long long *thi, int *bad,
@@ -1795,14 +1795,14 @@ __device__ __forceinline__ void deposit_pairs32(const DepositArgs &a, int axis, 
     const int chunk = a.chunk;
     const float bintov_f = (float)bintov_d;
     const Setup32 k32(a.lp, bintov_d);
-    for (;;) {
+    for (unsigned mine = 0;; mine++) {
         unsigned c = 0;
         if (lane == 0)
             c = atomicAdd(s_chunk, 1u);
         c = __shfl_sync(0xffffffffu, c, 0);
         const long long cb = e0 + (long long)c * chunk;
         if (cb >= e1)
-            break;
+            return mine;
         const int n = (int)min((long long)chunk, e1 - cb);
         const PairRec *rec = REC ? reinterpret_cast<const PairRec *>(a.pl.rec) : nullptr;
         if constexpr (REC) {
@@ -1923,6 +1923,36 @@ __device__ __forceinline__ void deposit_pairs_col32(const DepositArgs &a, int ax
             }
         }
         __syncwarp();
+    }
+}
+
+// The FP32 form's sums to the output row (whole block): pixels, plus the
+// interpolant of their tile's node sums (converted in place) in the first `ntiles`
+// tiles.
+__device__ __forceinline__ void split32_flush(double *row, int nbins, int ntiles,
+                                              const unsigned long long *lo,
+                                              const unsigned long long *hi,
+                                              unsigned long long *tlo, unsigned long long *thi,
+                                              int S)
+{
+    double *node = reinterpret_cast<double *>(tlo);
+    if (ntiles) {
+        for (int j = threadIdx.x; j < ntiles * TILE_M; j += blockDim.x)
+            node[j] = from_split(tlo[j], thi[j], S);
+        __syncthreads();
+    }
+    for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
+        double v = from_split(lo[j], hi[j], S);
+        if (j < ntiles * TILE_W) {
+            const double *w = g_tile.w + (j % TILE_W) * TILE_M;
+            const double *nd = node + (j / TILE_W) * TILE_M;
+            double f = 0.0;
+#pragma unroll
+            for (int m = 0; m < TILE_M; m++)
+                f = fma(w[m], nd[m], f);
+            v += f;
+        }
+        row[j] = v;
     }
 }
 
@@ -2069,29 +2099,11 @@ __global__ void __launch_bounds__(MAXT, 1)
                 a.bad_lines[atomicAdd(a.n_bad, 1)] = line;
         } else if (B > 0.0) {
             double *row = a.out + (size_t)line * nbins;
-            if (tlo) {
-                // node sums to double in place, then pixel + its tile's interpolant
-                double *node = reinterpret_cast<double *>(tlo);
-                for (int j = threadIdx.x; j < nnodes; j += blockDim.x)
-                    node[j] = from_split(tlo[j], thi[j], S);
-                __syncthreads();
-                for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
-                    double v = from_split(lo[j], hi[j], S);
-                    if (j < ntiles * TILE_W) {
-                        const double *w = g_tile.w + (j % TILE_W) * TILE_M;
-                        const double *nd = node + (j / TILE_W) * TILE_M;
-                        double f = 0.0;
-#pragma unroll
-                        for (int m = 0; m < TILE_M; m++)
-                            f = fma(w[m], nd[m], f);
-                        v += f;
-                    }
-                    row[j] = v;
-                }
-            } else {
+            if constexpr (PREC == 1)
+                split32_flush(row, nbins, tlo ? ntiles : 0, lo, hi, tlo, thi, S);
+            else
                 for (int j = threadIdx.x; j < nbins; j += blockDim.x)
-                    row[j] = PREC == 0 ? from_fixed(lo[j], hi[j], S) : from_split(lo[j], hi[j], S);
-            }
+                    row[j] = from_fixed(lo[j], hi[j], S);
         }
         if (!a.persistent)
             break;
@@ -2110,6 +2122,127 @@ __global__ void __launch_bounds__(MAXT, 1)
         atomicAdd(&a.counters[5], ct.e);
         atomicAdd(&a.counters[6], ct.f);
         atomicAdd(&a.counters[7], ct.g);
+    }
+}
+
+// The FP32 optical depth when there are fewer sightlines than SMs: blocks share
+// sightlines as in fast64_kernel (an owner forms the bound, then chunks of pairs go
+// to every block that joins; a helper's sums are merged in global memory, and the
+// block that completes the sightline writes it).  The sums are integers, so the
+// bits are those of deposit_kernel.  48^3 particles, 33 sightlines x 1115 pixels,
+// 152 SMs: 495 us with a block per sightline, 143 us so.
+constexpr int SPLIT32_THREADS = 1024, SPLIT32_CHUNK = 8;
+
+__global__ void __launch_bounds__(SPLIT32_THREADS, 1) split32_kernel(DepositArgs a)
+{
+    extern __shared__ __align__(16) unsigned long long smem[];
+    __shared__ BoundScratch red;
+    __shared__ float2 vtab[FSG_V32_N];
+    __shared__ unsigned long long s_best;
+    __shared__ int s_bad;
+    __shared__ unsigned s_ticket, s_mine, s_last;
+    const int nbins = a.lp.nbins;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double bintov_d = a.lp.vbox / nbins;
+    stage_voigt32(vtab);
+    const Bound32 bk(a.lp);
+    // dynamic shared memory: [accumulators lo, hi] [pair staging] [tile nodes lo, hi]
+    unsigned long long *lo = smem, *hi = smem + nbins;
+    Stage32 *stage = reinterpret_cast<Stage32 *>(smem + 2 * (size_t)nbins);
+    const int ntiles = a.tiles ? nbins / TILE_W : 0;
+    const int nnodes = ntiles * TILE_M;
+    unsigned long long *tlo =
+        nnodes ? reinterpret_cast<unsigned long long *>(stage + (SPLIT32_THREADS / 32) * a.chunk)
+               : nullptr;
+    unsigned long long *thi = nnodes ? tlo + nnodes : nullptr;
+    const SplitState sp = split_state(a.split_ws, a.nlos, nbins, nnodes);
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0)
+            s_ticket = atomicAdd(a.ticket, 1u);
+        __syncthreads();
+        int q = (int)min(s_ticket, 0x7fffffffu);
+        const bool owner = q < a.nlos;
+        if (!owner) {
+            q = pick_line(a, sp, SPLIT32_THREADS / 32, &s_best);
+            if (q < 0)
+                break;
+        }
+        const int line = a.line_order[q];
+        const int axis = a.t.axis[line];
+        const long long e0 = a.pl.off[line], e1 = a.pl.off[line + 1];
+        const unsigned nchunks = (unsigned)((e1 - e0 + a.chunk - 1) / a.chunk);
+        double B;
+        if (owner) {
+            const auto bound = [&](long long e) {
+                return tau_pair_bound32(bk, load_pair(a.p, a.pl, e, axis, true, a.dev_err));
+            };
+            B = order_free_bound(e0, e1, bound, bound, &red);
+        } else {
+            B = __ldcg(&sp.B[q]);
+        }
+        const bool live = isfinite(B) && B > 0.0;
+        for (int j = threadIdx.x; j < 2 * nbins; j += SPLIT32_THREADS)
+            lo[j] = 0ull;
+        for (int j = threadIdx.x; j < 2 * nnodes; j += SPLIT32_THREADS)
+            tlo[j] = 0ull;
+        if (threadIdx.x == 0) {
+            s_mine = 0u;
+            s_bad = !isfinite(B);
+            if (owner) {
+                sp.B[q] = B;
+                __threadfence();
+                if (live)
+                    atomicExch(&sp.ready[q], 1u);
+                atomicAdd(sp.started, 1u);
+            }
+        }
+        __syncthreads();
+        const int S = live ? SPLIT_TOP - ilogb(B) : 0;
+        if (live) {
+            Counters ct{};
+            const unsigned n = deposit_pairs32<false, false>(
+                a, axis, e0, e1, S, lo, hi, tlo, thi, &s_bad, stage + warp * a.chunk,
+                &sp.next[q], vtab, bintov_d, lane, ct);
+            if (lane == 0 && n)
+                atomicAdd(&s_mine, n);
+        }
+        __syncthreads();
+        bool bad = s_bad != 0;
+        const unsigned mine = s_mine;
+        if (live && mine != nchunks) {
+            if (mine == 0u)
+                continue;
+            unsigned long long *g = sp.acc + (size_t)q * sp.words;
+            for (int j = threadIdx.x; j < 2 * nbins; j += SPLIT32_THREADS)
+                if (lo[j])
+                    atomicAdd(g + j, lo[j]);
+            for (int j = threadIdx.x; j < 2 * nnodes; j += SPLIT32_THREADS)
+                if (tlo[j])
+                    atomicAdd(g + 2 * (size_t)nbins + j, tlo[j]);
+            if (threadIdx.x == 0 && bad)
+                atomicOr(&sp.bad[q], 1u);
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0)
+                s_last = atomicAdd(&sp.done[q], mine) + mine == nchunks;
+            __syncthreads();
+            if (!s_last)
+                continue;
+            __threadfence();
+            for (int j = threadIdx.x; j < 2 * nbins; j += SPLIT32_THREADS)
+                lo[j] = __ldcg(g + j);
+            for (int j = threadIdx.x; j < 2 * nnodes; j += SPLIT32_THREADS)
+                tlo[j] = __ldcg(g + 2 * (size_t)nbins + j);
+            bad = ld_cg(&sp.bad[q]) != 0u;
+            __syncthreads();
+        }
+        if (bad) {
+            if (threadIdx.x == 0)
+                a.bad_lines[atomicAdd(a.n_bad, 1)] = line;
+        } else if (live) {
+            split32_flush(a.out + (size_t)line * nbins, nbins, ntiles, lo, hi, tlo, thi, S);
+        }
     }
 }
 
@@ -3106,20 +3239,41 @@ int fast64_threads(int compute_tau) { return compute_tau ? T64_THREADS : C64_THR
 // pairs in chunks of 8 leave a third of the warps without one).
 void deposit_fit_chunk(DepositLaunch &cfg, long long npairs, int sms)
 {
+    for (cfg.split32 = cfg.split32 ? SPLIT32_CHUNK : 0;
+         cfg.split32 > 2 && npairs < 4ll * sms * (SPLIT32_THREADS / 32) * cfg.split32;)
+        cfg.split32 /= 2;
     if (!cfg.fast64)
         return;
     while (cfg.chunk > 2 && npairs < 4ll * sms * (cfg.threads / 32) * cfg.chunk)
         cfg.chunk /= 2;
 }
 
+namespace {
+DepositLaunch split32_launch(const DepositLaunch &cfg)
+{
+    DepositLaunch c = cfg;
+    c.threads = SPLIT32_THREADS;
+    c.chunk = cfg.split32;
+    return c;
+}
+size_t split32_smem(const DepositLaunch &cfg, int nbins)
+{
+    return deposit_smem_bytes(split32_launch(cfg), 1, nbins);
+}
+}  // namespace
+
 // Blocks help each other's sightlines (fast64_kernel) while a block has few of
 // them, 8 on average: beyond that the queue's tail is short against the whole,
 // and the words in global memory would grow (16 bytes a pixel and tile node of
 // every sightline; at most SPLIT_MAX bytes).  Also for nonpersistent launches:
-// never.
+// never.  FP32 optical depths (split32_kernel): fewer sightlines than SMs, where
+// whole SMs would stay idle.
 size_t deposit_split_bytes(const DepositLaunch &cfg, int nbins, int nlos, int sms)
 {
     constexpr size_t SPLIT_MAX = (size_t)1 << 29;
+    if (cfg.split32 && cfg.smem_mode && nlos < sms &&
+        split32_smem(cfg, nbins) <= (size_t)(max_smem_optin() - STATIC_SMEM_RESERVE))
+        return split_bytes(nlos, nbins, cfg.tiles ? TILE_M * (nbins / TILE_W) : 0);
     if (!cfg.fast64 || !cfg.smem_mode || !cfg.persistent || nlos > 8 * sms)
         return 0;
     const size_t b = split_bytes(nlos, nbins, tiles64_layout(cfg.tiles, nbins).nodes);
@@ -3180,6 +3334,19 @@ int launch_deposit(const LineParams &lp, const LineTables &t, const Particles &p
                             split_bytes(nlos, lp.nbins,
                                         tiles64_layout(cfg.tiles, lp.nbins).nodes), s);
         k<<<cfg.persistent ? cfg.grid : nlos, cfg.threads, smem, s>>>(a);
+        return launched;
+    }
+    if (cfg.split32 && cfg.split_ws && counters == nullptr) {
+        const size_t bytes = split32_smem(cfg, lp.nbins);
+        a.split_ws = cfg.split_ws;
+        a.chunk = cfg.split32;
+        a.pl.rec = nullptr;
+        cudaFuncSetAttribute(split32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)bytes);
+        cudaMemsetAsync(a.split_ws, 0,
+                        split_bytes(nlos, lp.nbins,
+                                    cfg.tiles ? TILE_M * (lp.nbins / TILE_W) : 0), s);
+        split32_kernel<<<cfg.grid, SPLIT32_THREADS, bytes, s>>>(a);
         return launched;
     }
     const int grid = cfg.persistent ? cfg.grid : nlos;

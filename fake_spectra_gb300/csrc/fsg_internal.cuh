@@ -307,7 +307,10 @@ struct DepositLaunch {
     int rec;                 // FP32 tau: through pair records (PairLists::rec must be set)
     int fast64;              // FP64 through fast64_kernel (planned with smem_mode)
     int table;               // fast64_kernel, tau: K table staged in shared memory
-    void *split_ws;          // fast64_kernel: deposit_split_bytes() of device memory, or null
+    int split32;             // FP32 tau: may share sightlines between blocks; after
+                             // deposit_fit_chunk the pairs staged per warp then
+    void *split_ws;          // shared sightlines: deposit_split_bytes() of device memory, or
+                             // null
 };
 
 // Deposits all pairs of all sightlines into out[L*nbins] (pre-zeroed).  Lines

@@ -304,6 +304,7 @@ int noalloc_run(int compute_tau, int nbins, int kernel, double box, double velfa
         cfg.threads = threads;
         cfg.tiles = 1;
         cfg.fast64 = precision == FSG_PREC_FP64;
+        cfg.split32 = precision == FSG_PREC_FP32 && compute_tau;
         if (cfg.fast64) {
             cfg.threads = fast64_threads(compute_tau);
             deposit_plan(cfg, compute_tau, nbins);
@@ -324,7 +325,7 @@ int noalloc_run(int compute_tau, int nbins, int kernel, double box, double velfa
         const size_t sb = deposit_split_bytes(cfg, nbins, nlos, sms);
         if (sb && (size_t)(pair_cap - total) * 8 >= sb + 256) {
             cfg.split_ws = (void *)(((uintptr_t)(d_dr2 + total) + 255) & ~(uintptr_t)255);
-            cfg.grid = sms * per_sm;
+            cfg.grid = sms * (cfg.split32 ? 1 : per_sm);
         }
         PairLists pl{d_off, d_part, d_dr2};
         NA_CUDA(cudaMemsetAsync(d_ticket, 0, 4, s), "memset");
