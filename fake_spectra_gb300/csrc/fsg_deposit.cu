@@ -2125,7 +2125,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
 }
 
-// The FP32 optical depth when there are fewer sightlines than SMs: blocks share
+// The FP32 optical depth when there are few sightlines per SM: blocks share
 // sightlines as in fast64_kernel (an owner forms the bound, then chunks of pairs go
 // to every block that joins; a helper's sums are merged in global memory, and the
 // block that completes the sightline writes it).  The sums are integers, so the
@@ -3266,12 +3266,14 @@ size_t split32_smem(const DepositLaunch &cfg, int nbins)
 // them, 8 on average: beyond that the queue's tail is short against the whole,
 // and the words in global memory would grow (16 bytes a pixel and tile node of
 // every sightline; at most SPLIT_MAX bytes).  Also for nonpersistent launches:
-// never.  FP32 optical depths (split32_kernel): fewer sightlines than SMs, where
-// whole SMs would stay idle.
+// never.  FP32 optical depths (split32_kernel): up to 3 sightlines per SM, where
+// SMs idle (192^3 particles, 11152 pixels, 152 SMs, ms of deposit without | with
+// sharing: 160 sightlines 8.0 | 3.8, 305 9.7 | 7.0, 460 10.2 | 9.8, 620 13.4 | 13.2,
+// 900 18.9 | 19.7).
 size_t deposit_split_bytes(const DepositLaunch &cfg, int nbins, int nlos, int sms)
 {
     constexpr size_t SPLIT_MAX = (size_t)1 << 29;
-    if (cfg.split32 && cfg.smem_mode && nlos < sms &&
+    if (cfg.split32 && cfg.smem_mode && nlos <= 3 * sms &&
         split32_smem(cfg, nbins) <= (size_t)(max_smem_optin() - STATIC_SMEM_RESERVE))
         return split_bytes(nlos, nbins, cfg.tiles ? TILE_M * (nbins / TILE_W) : 0);
     if (!cfg.fast64 || !cfg.smem_mode || !cfg.persistent || nlos > 8 * sms)

@@ -10,7 +10,7 @@ from fake_spectra_gb300 import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nlos", [1, 5, 120])
+@pytest.mark.parametrize("nlos", [1, 5, 120, 400])
 @pytest.mark.parametrize("nbins", [50, 1115, 9000])
 def test_same_bits(ctx, nlos, nbins):
     import torch
