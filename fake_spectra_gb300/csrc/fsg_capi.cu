@@ -979,11 +979,19 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
         p.dens = dens[k];
         apply_tuning(c, lps[k], opt, p, pl, outs[k], cfgs.back());
     }
-    for (const DepositLaunch &cf : cfgs)
+    // the forms differ in what they need: the shared-sightline buffer may have grown
+    // after an earlier deposit's plan named it, and any of them may accumulate in
+    // global memory
+    bool global_acc = false;
+    for (DepositLaunch &cf : cfgs) {
         if (cf.rec)
             pl.rec = c->ensure(c->prec, 32 * (size_t)c->npairs);
+        if (cf.split_ws)
+            cf.split_ws = c->split.p;
+        global_acc = global_acc || !cf.smem_mode;
+    }
     unsigned long long *gacc = nullptr;
-    if (!cfgs[0].smem_mode)
+    if (global_acc)
         gacc = (unsigned long long *)c->ensure(c->gacc, sizeof(unsigned long long) * 2 * nout);
     auto *ticket = (unsigned *)c->ensure(c->ticket, sizeof(unsigned));
     auto *bad = (int *)c->ensure(c->bad, sizeof(int) * nlos);
@@ -1028,6 +1036,7 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
         put(cfgs[k].chunk);
         put(cfgs[k].tiles);
         put(cfgs[k].rec);
+        put(cfgs[k].split32);
         putp(cfgs[k].split_ws);
     }
     cudaStream_t s = c->own;
@@ -1807,7 +1816,7 @@ int fsg_colden_channels_device(fsg_context *ctx, int nbins, int kernel, double b
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         const int grid = std::min(nlos, sms * plan.per_sm);
         unsigned long long *gacc = nullptr;
-        if (!plan.smem_mode)
+        if (plan.smem_rows < 2 * nch)
             gacc = (unsigned long long *)ctx->ensure(
                 ctx->gacc, sizeof(unsigned long long) * plan.acc_words_per_cta * grid);
         auto *bad = (int *)ctx->ensure(ctx->bad, sizeof(int) * (size_t)nch * nlos);
