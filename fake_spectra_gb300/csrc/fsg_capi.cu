@@ -1816,7 +1816,7 @@ int fsg_colden_channels_device(fsg_context *ctx, int nbins, int kernel, double b
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         const int grid = std::min(nlos, sms * plan.per_sm);
         unsigned long long *gacc = nullptr;
-        if (plan.smem_rows < 2 * nch)
+        if (!plan.smem_mode)
             gacc = (unsigned long long *)ctx->ensure(
                 ctx->gacc, sizeof(unsigned long long) * plan.acc_words_per_cta * grid);
         auto *bad = (int *)ctx->ensure(ctx->bad, sizeof(int) * (size_t)nch * nlos);
