@@ -2799,7 +2799,7 @@ __device__ __forceinline__ GradSums grad_far(const StageGrad &g, float V)
 // far-field tiles, the transpose of that, the pair's value at each node times
 // the node's share of dL/dtau (grow: the row's pixels, gnode: its nodes; gnode
 // null: every pixel).  128^3, 1024 sightlines x 1115 pixels: 8.66 ms with all
-// seven nodes at every pixel of the window, 5.4 ms so.
+// seven nodes at every pixel of the window, 5.3 ms so.
 __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, const float *grow,
                                             const float *gnode, int nbins, float tautail,
                                             int lane, const float2 *vtab, float &ad, float &av,
@@ -2808,79 +2808,64 @@ __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, 
     const int half = nbins / 2;
     const int j0 = s.j0;
     const float lane_f = (float)lane;
-    const float dmin = fmaxf(s.vmp, TILE_DIST * s.vk);
-    float vsure = -1.f;
+    const int np = s.npoints;
     ad = av = at = 0.f;
     for (int dir = 0; dir < 2; dir++) {
-        bool far = false, tiles = s.tiles && gnode != nullptr;
-        int k = 0, n = 0, items = 0, base = 0, jb_run = 0;
+        // the distance from which tiles are tried (infinite: no more)
+        float dmin = s.tiles && gnode != nullptr ? fmaxf(s.vmp, TILE_DIST * s.vk) : INFINITY;
+        int k = 0, items = 0, base = 0, jb_run = 0;
         while (k < half) {
             const int koff0 = dir == 0 ? k : -1 - k;
             const float kf0 = (float)koff0;
             int len = 32;
-            if (items == 0 && tiles) {
-                if (!far) {
-                    const float ve = dir == 0 ? fmaf(kf0, s.vk, s.v0) : -fmaf(kf0 + 1.f, s.vk, s.v0);
-                    far = ve >= dmin;
-                }
-                if (far) {
-                    const int jb = bin_from(j0, koff0, nbins);
-                    const int rem = dir == 0 ? (TILE_W - jb % TILE_W) % TILE_W
-                                             : (jb + 1) % TILE_W;
-                    if (vsure < 0.f)
-                        vsure = 0.999f * far_stop_radius(s, tautail);
+            if (items == 0 &&
+                (dir == 0 ? fmaf(kf0, s.vk, s.v0) : -fmaf(kf0 + 1.f, s.vk, s.v0)) >= dmin) {
+                const int jb = bin_from(j0, koff0, nbins);
+                const int rem = dir == 0 ? (TILE_W - jb % TILE_W) % TILE_W : (jb + 1) % TILE_W;
+                // the next tile is inside the window when its last pixel's value, taken
+                // 0.11% farther out, is above tautail
+                const float kt = (float)(k + rem) + (float)(TILE_W - 1);
+                const float ve = dir == 0 ? fmaf(kt, s.vk, s.vmid0)
+                                          : fmaf(kt + 1.f, s.vk, -s.vmid0);
+                if (half - k - rem < TILE_W ||
+                    !(s.scale * grad_far(g, 1.0011f * ve).d >= tautail)) {
+                    dmin = INFINITY;       // the window ends before the next tile does
+                } else if (rem == 0) {
+                    const float vsure = 0.999f * far_stop_radius(s, tautail);
                     const float klim = dir == 0 ? (vsure - s.vmid0) / s.vk
                                                 : (vsure + s.vmid0) / s.vk - 1.f;
-                    if (!(klim >= (float)(k + rem) + (float)(TILE_W - 1)) ||
-                        half - k - rem < TILE_W) {
-                        tiles = false;     // the window ends before the next tile does
-                    } else if (rem == 0) {
-                        n = 0;
-                        if (klim >= (float)k + (float)(TILE_W - 1))
-                            n = (int)fminf((klim - (float)k + 1.f) / (float)TILE_W, 1e6f);
-                        n = min(n, (half - k) / TILE_W);
-                        n = min(n, dir == 0 ? (nbins - jb) / TILE_W : (jb + 1) / TILE_W);
-                        if (n > 0) {
-                            items = n * TILE_M;
-                            base = 0;
-                            jb_run = jb;
-                        } else {
-                            tiles = dir == 0 ? (nbins - jb < TILE_W) : false;
-                        }
-                    } else {
-                        len = min(32, rem);
+                    int n = (int)fminf((klim - (float)k + 1.f) / (float)TILE_W, 1e6f);
+                    n = min(n, (half - k) / TILE_W);
+                    n = min(n, dir == 0 ? (nbins - jb) / TILE_W : (jb + 1) / TILE_W);
+                    if (n > 0) {
+                        items = n * TILE_M;
+                        base = 0;
+                        jb_run = jb;
+                    } else if (dir != 0 || nbins - jb >= TILE_W) {
+                        dmin = INFINITY;
                     }
+                } else {
+                    len = min(32, rem);
                 }
             }
-            // one evaluation per lane: a tile node or a pixel, and its dL/dtau; the
-            // position is x mul (mul: to units of b) plus the sample's offset
-            float x, mul = 1.f, gg = 0.f;
-            bool on;
+            // one evaluation per lane: a tile node or a pixel; the position is x mul
+            // (mul: to units of b) plus the sample's offset
+            float x, mul = 1.f;
             if (items) {
-                const int it0 = base + lane;
-                on = it0 < items;
-                const int it = on ? it0 : 0;
+                const int it = min(base + lane, items - 1);
                 const int t = it / TILE_M, m = it - t * TILE_M;
                 const int kt = k + TILE_W * t;
                 x = fmaf((float)(dir == 0 ? kt : -kt - TILE_W), s.vk, s.v0);
                 x = fmaf(g_tile.x[m], s.vk, x);
-                if (on)
-                    gg = gnode[(dir == 0 ? jb_run + TILE_W * t
-                                         : jb_run - TILE_W * (t + 1) + 1) / TILE_W * TILE_M + m];
             } else {
-                const int kk = k + lane;
-                on = lane < len && kk < half;
                 x = fmaf(dir == 0 ? kf0 + lane_f : kf0 - lane_f, s.bintov, s.base0);
                 mul = s.inv_b;
-                if (on)
-                    gg = grow[bin_from(j0, dir == 0 ? kk : -1 - kk, nbins)];
             }
             // The stop rule compares with tautail: where the wing polynomial comes
             // within 1e-4 of it (its own error is 1e-6) the node sums decide.  A stop
             // one pixel off moves the temperature gradient of a weak particle, whose
             // window ends on its Gaussian flank, by 1e-3 of the largest.
             GradSums r;
-            const int np = s.npoints;
             bool nodes = false;
             do {
                 bool poly = false;
@@ -2898,26 +2883,37 @@ __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, 
                     poly |= wing;
                 }
                 nodes = poly && !items &&
-                        __any_sync(0xffffffffu, on && fabsf(fmaf(s.scale, r.d, -tautail)) <=
-                                                          1e-4f * tautail);
+                        __any_sync(0xffffffffu, fabsf(fmaf(s.scale, r.d, -tautail)) <=
+                                                    1e-4f * tautail);
             } while (nodes);
-            unsigned msk = 0;
-            if (!items) {
-                msk = __ballot_sync(0xffffffffu, on && s.scale * r.d < tautail);
-                on = on && lane <= (msk ? __ffs(msk) - 1 : 31);
-            }
-            if (on) {
-                ad = fmaf(gg, r.d, ad);
-                av = fmaf(gg, r.v, av);
-                at = fmaf(gg, r.t, at);
-            }
+            // times dL/dtau of the pixel, or the node's share of it
             if (items) {
+                const int it = base + lane;
+                if (it < items) {
+                    const int t = it / TILE_M;
+                    const float gg = gnode[(dir == 0 ? jb_run + TILE_W * t
+                                                     : jb_run - TILE_W * (t + 1) + 1) / TILE_W *
+                                               TILE_M + it - t * TILE_M];
+                    ad = fmaf(gg, r.d, ad);
+                    av = fmaf(gg, r.v, av);
+                    at = fmaf(gg, r.t, at);
+                }
                 base += 32;
                 if (base >= items) {
-                    k += TILE_W * n;
+                    k += TILE_W * (items / TILE_M);
                     items = 0;
                 }
                 continue;
+            }
+            const int kk = k + lane;
+            bool on = lane < len && kk < half;
+            const unsigned msk = __ballot_sync(0xffffffffu, on && s.scale * r.d < tautail);
+            on = on && lane <= (msk ? __ffs(msk) - 1 : 31);
+            if (on) {
+                const float gg = grow[bin_from(j0, dir == 0 ? kk : -1 - kk, nbins)];
+                ad = fmaf(gg, r.d, ad);
+                av = fmaf(gg, r.v, av);
+                at = fmaf(gg, r.t, at);
             }
             if (msk)
                 break;
@@ -2961,13 +2957,21 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
             grow[j] = (float)gt[j];
         if (threadIdx.x == 0)
             s_chunk = 0u;
-        for (int j = threadIdx.x; j < nnodes; j += blockDim.x) {
+        // eight lanes per node (one lane's chain of 64 FP64 FMAs left the SM waiting)
+        static_assert(TILE_M * 8 % 32 == 0, "whole warps");
+        for (int q = threadIdx.x; q < 8 * nnodes; q += blockDim.x) {
+            const int j = q >> 3;
             const double *row = gt + j / TILE_M * TILE_W;
             const double *w = g_tile.w + j % TILE_M;
             double sum = 0.0;
-            for (int p = 0; p < TILE_W; p++)
-                sum = fma(w[p * TILE_M], row[p], sum);
-            gnode[j] = (float)sum;
+#pragma unroll
+            for (int p = 0; p < TILE_W; p += 8)
+                sum = fma(w[(p + (q & 7)) * TILE_M], row[p + (q & 7)], sum);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1)
+                sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if ((q & 7) == 0)
+                gnode[j] = (float)sum;
         }
         __syncthreads();
         for (;;) {
