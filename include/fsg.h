@@ -34,7 +34,7 @@ typedef enum {
 
 /* Arithmetic form of the deposit. */
 typedef enum {
-    FSG_PREC_FP64 = 0, /* plain form: FP64 everywhere (the drop-in default) */
+    FSG_PREC_FP64 = 0, /* plain form: FP64 results (the drop-in default)    */
     FSG_PREC_FP32 = 1  /* tuned form: FP32 profile/kernel arithmetic        */
 } fsg_precision;
 
@@ -47,7 +47,7 @@ typedef struct {
     int count_work; /* 1 = run the counting variant of the deposit and report
                        the algorithmic work in fsg_stats (slower; for the
                        roofline only)                                         */
-    int no_far_tiles; /* FP32 tau: 1 = deposit the far damping wing pixel by
+    int no_far_tiles; /* tau: 1 = deposit the far damping wing pixel by
                        pixel; 0 (default) = through per-tile Chebyshev nodes
                        where the node accumulators fit on chip               */
     int chunk;      /* FP32 form: sightline-particle pairs staged per warp
@@ -219,8 +219,8 @@ int fsg_mean_flux_scale_device(fsg_context *ctx, const double *tau, int64_t n,
 int fsg_mean_flux_device(fsg_context *ctx, const double *tau, int64_t n, double scale,
                          double *mean, char *errbuf, size_t errlen);
 
-/* out[i] = exp(y[i]) (y, out DEVICE, n doubles) with the FP64 exponential the
- * mean-flux and flux-power passes use (table-driven, within about one ulp of
+/* out[i] = exp(y[i]) (y, out DEVICE, n doubles) with the exponential the
+ * mean-flux and flux-power passes use (in integers, within about one ulp of
  * exp); exposed so that its accuracy can be checked. */
 int fsg_flux_exp_device(fsg_context *ctx, const double *y, int64_t n, double *out, char *errbuf,
                         size_t errlen);
