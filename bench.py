@@ -86,9 +86,9 @@ def search_roofline(npart, npairs, nlos, ms):
     achieved = algo / (ms * 1e-3) / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": hbm, "peak_source": src,
             "unit": "GB/s", "frac": achieved / hbm, "bytes": algo,
-            "note": "the search is limited by the cell walk (latency of the dependent cell "
-                    "and sightline loads), not by HBM (16 B of particle data per particle "
-                    "per pass); the FP64 predicate runs only on the thin shell the float "
+            "note": "the search is limited by instruction issue and the candidates' dependent "
+                    "loads, not by HBM (16 B of particle data per particle per pass); the "
+                    "FP64 predicate runs only on the thin shell the float "
                     "tests cannot decide"}
 
 
@@ -649,7 +649,7 @@ def main():
                      "executed": {"flops_per_eval_by_branch": FLOPS_FP32,
                                   "achieved": achieved_exec, "frac": achieved_exec / peak32,
                                   "note": "flops of the pixel-by-pixel walk over the same "
-                                          "windows; far-field tiles execute fewer (10 node "
+                                          "windows; far-field tiles execute fewer (8 node "
                                           "evaluations per 64 far pixels), so this is an upper "
                                           "bound of the executed rate"},
                      "peak_fp64": peak64,

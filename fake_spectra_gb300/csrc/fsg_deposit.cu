@@ -6,8 +6,9 @@
 //
 // Work decomposition: one CTA owns one sightline at a time (sightlines are
 // visited in descending pair count, either one CTA per sightline or resident
-// CTAs draining a ticket queue); each warp takes one (particle, sightline)
-// pair at a time and walks its pixel window 32 pixels per step.
+// CTAs draining a ticket queue; few sightlines are shared between CTAs); each warp
+// takes one (particle, sightline) pair at a time and walks its pixel window 32
+// pixels per step.
 // tau: forward from zmax and backward from zmax-1, each direction stopping
 // after the first pixel whose contribution is below tautail (that pixel is
 // still added) or after nbins/2 pixels, exactly the rule of
@@ -15,7 +16,9 @@
 // colden: the fixed pixel range of absorption.cpp:190-209.
 //
 // Two arithmetic forms share this skeleton:
-//   FP64 (plain): every quantity in double, as the reference computes it.
+//   FP64 (plain): fast64_kernel (fsg_fast64.cuh), double where the reference's
+//     rounding decides and 64-bit integers elsewhere; the walk here, every quantity
+//     in double, serves the counting variant and rows without room for its staging.
 //   FP32 (tuned): profile, kernel and pixel arithmetic in float; double only
 //     for the particle velocity, the bin of the particle (zmax) and the offset
 //     of the first pixel from it, so box-sized coordinates lose nothing.  Far
