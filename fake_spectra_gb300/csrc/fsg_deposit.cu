@@ -36,6 +36,7 @@
 // (inf/NaN inputs) are re-run by a plain FP64-atomic fallback so that inf/NaN
 // propagate as they do in the reference.
 #include "fsg_internal.cuh"
+#include "fsg_share.cuh"
 #include "fsg_voigt.cuh"
 #include "fsg_voigt_fix.cuh"
 #include "fsg_spline_fix.cuh"
@@ -2192,13 +2193,8 @@ __global__ void __launch_bounds__(SPLIT32_THREADS, 1) split32_kernel(DepositArgs
         if (threadIdx.x == 0) {
             s_mine = 0u;
             s_bad = !isfinite(B);
-            if (owner) {
-                sp.B[q] = B;
-                __threadfence();
-                if (live)
-                    atomicExch(&sp.ready[q], 1u);
-                atomicAdd(sp.started, 1u);
-            }
+            if (owner)
+                share_open(sp, q, B, live);
         }
         __syncthreads();
         const int S = live ? SPLIT_TOP - ilogb(B) : 0;
@@ -2225,19 +2221,17 @@ __global__ void __launch_bounds__(SPLIT32_THREADS, 1) split32_kernel(DepositArgs
                     atomicAdd(g + 2 * (size_t)nbins + j, tlo[j]);
             if (threadIdx.x == 0 && bad)
                 atomicOr(&sp.bad[q], 1u);
-            __threadfence();
             __syncthreads();
             if (threadIdx.x == 0)
-                s_last = atomicAdd(&sp.done[q], mine) + mine == nchunks;
+                s_last = share_done(sp, q, mine, nchunks);
             __syncthreads();
             if (!s_last)
                 continue;
-            __threadfence();
             for (int j = threadIdx.x; j < 2 * nbins; j += SPLIT32_THREADS)
                 lo[j] = __ldcg(g + j);
             for (int j = threadIdx.x; j < 2 * nnodes; j += SPLIT32_THREADS)
                 tlo[j] = __ldcg(g + 2 * (size_t)nbins + j);
-            bad = ld_cg(&sp.bad[q]) != 0u;
+            bad = __ldcg(&sp.bad[q]) != 0u;
             __syncthreads();
         }
         if (bad) {

@@ -12,45 +12,6 @@
 // left the SMs idle for 69% of the kernel, and 37% with a cluster of four
 // blocks per sightline.)
 
-// Per-launch state of shared sightlines, zeroed before the launch.
-struct SplitState {
-    unsigned *next, *done;   // [nlos] chunks taken, chunks whose sums are in acc
-    unsigned *ready;         // [nlos] B is set and chunks may be taken
-    unsigned *active;        // [nlos] blocks that have joined (a hint)
-    unsigned *bad;           // [nlos] a contribution was not finite
-    unsigned *started;       // sightlines that are ready or need no chunks
-    double *B;               // [nlos] bound of the sightline total
-    unsigned long long *acc;     // [nlos][2 (nbins + nodes)]
-    size_t words;            // 2 (nbins + nodes)
-};
-
-size_t split_bytes(int nlos, int nbins, int nodes)
-{
-    return 64 + (size_t)nlos * (5 * sizeof(unsigned) + sizeof(double) + 4 +
-                                sizeof(unsigned long long) * 2 * ((size_t)nbins + nodes));
-}
-
-__host__ __device__ inline SplitState split_state(void *ws, int nlos, int nbins, int nodes)
-{
-    SplitState st;
-    st.words = 2 * ((size_t)nbins + nodes);
-    unsigned char *p = (unsigned char *)ws;
-    st.acc = (unsigned long long *)p;
-    p += sizeof(unsigned long long) * st.words * nlos;
-    st.B = (double *)p;
-    p += sizeof(double) * nlos;
-    unsigned *u = (unsigned *)p;
-    st.next = u;
-    st.done = u + nlos;
-    st.ready = u + 2 * (size_t)nlos;
-    st.active = u + 3 * (size_t)nlos;
-    st.bad = u + 4 * (size_t)nlos;
-    st.started = u + 5 * (size_t)nlos;
-    return st;
-}
-
-__device__ __forceinline__ unsigned ld_cg(const unsigned *p) { return __ldcg(p); }
-
 // The sightline with the most chunks left per block working on it, or -1 (whole
 // block).  Waits a while for sightlines whose bound is still being formed: at
 // most SPLIT_POLLS polls, after which the block leaves (the owners need no help).
@@ -59,21 +20,21 @@ __device__ int pick_line(const DepositArgs &a, const SplitState &sp, unsigned mi
                          unsigned long long *s_best)
 {
     for (int poll = 0; poll < SPLIT_POLLS; poll++) {
-        const bool all = ld_cg(sp.started) >= (unsigned)a.nlos;
+        const bool all = share_all_open(sp, a.nlos);
         __syncthreads();
         if (threadIdx.x == 0)
             *s_best = 0ull;
         __syncthreads();
         for (int i = threadIdx.x; i < a.nlos; i += blockDim.x) {
             const int l = a.line_order[i];
-            if (!ld_cg(&sp.ready[i]))
+            if (!share_ready(sp, i))
                 continue;
             const long long n = (a.pl.off[l + 1] - a.pl.off[l] + a.chunk - 1) / a.chunk;
-            const long long left = n - (long long)ld_cg(&sp.next[i]);
+            const long long left = n - (long long)share_load(&sp.next[i]);
             if (left < (long long)min_left)
                 continue;
-            const unsigned score = (unsigned)min(left * 16 / (1 + (long long)ld_cg(&sp.active[i])),
-                                                 0x7fffffffll);
+            const long long blocks = 1 + (long long)share_load(&sp.active[i]);
+            const unsigned score = (unsigned)min(left * 16 / blocks, 0x7fffffffll);
             atomicMax(s_best, ((unsigned long long)score << 32) | (unsigned)(i + 1));
         }
         __syncthreads();
@@ -215,13 +176,8 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
             s_chunk = 0u;
             s_mine = 0u;
             s_bad = !isfinite(B);
-            if (owner && split) {
-                sp.B[q] = B;
-                __threadfence();
-                if (live)
-                    atomicExch(&sp.ready[q], 1u);
-                atomicAdd(sp.started, 1u);
-            }
+            if (owner && split)
+                share_open(sp, q, B, live);
         }
         __syncthreads();
         const int S = live ? 124 - ilogb(B) : 0;
@@ -265,14 +221,12 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
             merge(tlo, thi, 2 * (size_t)nbins, tl.nodes);
             if (threadIdx.x == 0 && bad)
                 atomicOr(&sp.bad[q], 1u);
-            __threadfence();
             __syncthreads();
             if (threadIdx.x == 0)
-                s_last = atomicAdd(&sp.done[q], mine) + mine == nchunks;
+                s_last = share_done(sp, q, mine, nchunks);
             __syncthreads();
             if (!s_last)
                 continue;
-            __threadfence();
             for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
                 lo[j] = __ldcg(g + j);
                 hi[j] = __ldcg(g + nbins + j);
@@ -281,7 +235,7 @@ __global__ void __launch_bounds__(TAU ? T64_THREADS : C64_THREADS, 1) fast64_ker
                 tlo[j] = __ldcg(g + 2 * (size_t)nbins + j);
                 thi[j] = __ldcg(g + 2 * (size_t)nbins + tl.nodes + j);
             }
-            bad = ld_cg(&sp.bad[q]) != 0u;
+            bad = __ldcg(&sp.bad[q]) != 0u;
             __syncthreads();
         }
         if (bad) {
