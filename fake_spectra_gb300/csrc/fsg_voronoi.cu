@@ -89,10 +89,13 @@ struct VorLine {
         const float *p = &a.pos[3 * (size_t)__ldg(&a.part[e0 + k])];
         return make_float3(__ldg(p + ax - 1), __ldg(p + i1), __ldg(p + i2));
     }
-    // float distance of a cell from the point x; shift is added along the sightline
+    // float distance of a cell from the point x, the part along the sightline changed
+    // by shift (to zero at least; NaN stays NaN).  The image of a cell outside the box
+    // has a negative distance, whose magnitude counts.
     __device__ __forceinline__ float dist(float3 q, float x, float shift) const
     {
-        const float dx = fmaxf(min_image_f(q.x - x, boxf) + shift, 0.f);
+        float dx = fabsf(min_image_f(q.x - x, boxf)) + shift;
+        dx = dx < 0.f ? 0.f : dx;
         const float dy = min_image_f(q.y - ypf, boxf), dz = min_image_f(q.z - zpf, boxf);
         return sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
     }
@@ -130,7 +133,7 @@ __device__ void gather_candidates(const VorArgs &a, const VorLine &L, float xm, 
     const float lim = ub + 2.f * L.margin(ub);
     for (int k = threadIdx.x; k < L.m; k += blockDim.x) {
         const float3 q = L.cell(a, k);
-        // NaN distances stay in, as candidates the comparisons below never pick
+        // NaN distances stay in: the comparisons of nearest_cell never pick them
         if (!(L.dist(q, xm, -w) > lim)) {
             const int i = atomicAdd(&sh.ncand, 1);
             if (i < VOR_CAND)
