@@ -2928,6 +2928,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
     extern __shared__ __align__(16) unsigned char gsmem[];
     __shared__ float2 vtab[FSG_V32_N];
     __shared__ unsigned s_ticket, s_chunk;
+    __shared__ int s_wild;
     stage_voigt32(vtab);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nbins = a.lp.nbins;
@@ -2941,8 +2942,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
                          : reinterpret_cast<float *>(gsmem + GRAD_STAGE);
     float *gnode = grow + nbins;
     const int nnodes = TILE_M * (nbins / TILE_W);
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
         s_ticket = atomicAdd(a.ticket, 1u);
+        s_wild = 0;
+    }
     __syncthreads();
     unsigned ticket = s_ticket;
     while (ticket < (unsigned)a.nlos) {
@@ -2950,8 +2953,12 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
         const int axis = a.t.axis[line];
         const double *gt = a.grad_tau + (size_t)line * nbins;
         const long long e0 = a.pl.off[line], e1 = a.pl.off[line + 1];
-        for (int j = threadIdx.x; j < nbins; j += blockDim.x)
-            grow[j] = (float)gt[j];
+        bool wild = false;       // a value or a node's share that is not finite as a float
+        for (int j = threadIdx.x; j < nbins; j += blockDim.x) {
+            const float g = (float)gt[j];
+            grow[j] = g;
+            wild = wild || !isfinite(g);
+        }
         if (threadIdx.x == 0)
             s_chunk = 0u;
         // eight lanes per node (one lane's chain of 64 FP64 FMAs left the SM waiting)
@@ -2967,9 +2974,13 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1)
                 sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            const float share = (float)sum;
+            wild = wild || !isfinite(share);
             if ((q & 7) == 0)
-                gnode[j] = (float)sum;
+                gnode[j] = share;
         }
+        if (wild)
+            s_wild = 1;
         __syncthreads();
         for (;;) {
             unsigned c = 0;
@@ -2988,6 +2999,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
                 g.pad = 0;
                 if (!stage32_setup(a.lp, k32, in, bintov_d, g.s, &g.scale_nod, g.D))
                     g.s.flags = STAGE_SKIP;
+                // the weights of a node have both signs: an infinity would become NaN,
+                // so such a row goes pixel by pixel
+                if (s_wild)
+                    g.s.flags &= ~STAGE_TILES;
                 sw[lane] = g;
             }
             __syncwarp();
@@ -3027,8 +3042,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
             __syncwarp();
         }
         __syncthreads();
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0) {
             s_ticket = atomicAdd(a.ticket, 1u);
+            s_wild = 0;
+        }
         __syncthreads();
         ticket = s_ticket;
     }
