@@ -100,7 +100,7 @@ struct fsg_context {
     DevBuf vseg, vscratch, vcofm;                            // Voronoi cells
     DevBuf tune_order;                                       // autotuner sample
     DevBuf prec;                                             // pair records (FP32 tau)
-    DevBuf split;                                            // shared sightlines (FP64)
+    DevBuf split;                                            // shared sightlines
     HostBuf hstage;   // host-pointer entries: pinned staging of inputs and output
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t cp[2] = {nullptr, nullptr};   // copy timing of the host-pointer entries
@@ -148,10 +148,38 @@ struct fsg_context {
             b.p = nullptr;
             b.cap = 0;
             size_t want = bytes + bytes / 8;
-            cuda_check(cudaMalloc(&b.p, want), "cudaMalloc");
+            cudaError_t e = cudaMalloc(&b.p, want);
+            if (e == cudaErrorMemoryAllocation && split.p) {
+                // the one buffer that a call can do without makes room
+                cudaGetLastError();
+                cuda_check(cudaFree(split.p), "cudaFree");
+                split = DevBuf{};
+                e = cudaMalloc(&b.p, want);
+            }
+            cuda_check(e, "cudaMalloc");
             b.cap = want;
         }
         return b.p;
+    }
+
+    // The buffer of shared sightlines, or null where it does not fit (what there is
+    // stays): the deposit then has a block per sightline.
+    void *ensure_split(size_t bytes)
+    {
+        if (split.cap < bytes) {
+            DevBuf b;
+            b.cap = bytes + bytes / 8;
+            const cudaError_t e = cudaMalloc(&b.p, b.cap);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            cuda_check(e, "cudaMalloc");
+            if (split.p)
+                cuda_check(cudaFree(split.p), "cudaFree");
+            split = b;
+        }
+        return split.p;
     }
 
     void *ensure_host(HostBuf &b, size_t bytes)
@@ -501,6 +529,7 @@ double mean_flux_of(fsg_context *c, const double *tau, long long n, double scale
 }
 
 DepositLaunch deposit_config(fsg_context *c, const LineParams &lp, const fsg_options *opt);
+void settle_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg);
 void apply_tuning(fsg_context *c, const LineParams &lp, const fsg_options *opt, const Particles &p,
                   PairLists pl, double *out, DepositLaunch &cfg);
 
@@ -550,15 +579,18 @@ void deposit(fsg_context *c, const LineParams &lp, const Particles &p, double *o
         ctr = (unsigned long long *)c->ensure(c->counters, sizeof(unsigned long long) * 8);
         cuda_check(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * 8, s), "memset");
     }
+    auto *ticket = (unsigned *)c->ensure(c->ticket, sizeof(unsigned) * fsg_context::ROW_GROUPS);
+    auto *bad = (int *)c->ensure(c->bad, sizeof(int) * nlos);
+    auto *nbad = (int *)c->ensure(c->nbad, sizeof(int));
+    auto *err = (unsigned *)c->ensure(c->err, sizeof(unsigned));
+    if (rows && rows->groups > 1)
+        c->ensure(c->gorder, sizeof(int) * (size_t)nlos);
+    settle_config(c, lp, cfg);
     // sightlines few enough to be shared between blocks are launched at once
     const int G = (rows && rows->groups > 1 && !count && !cfg.split_ws &&
                    nlos >= 64 * rows->groups)
                       ? std::min(rows->groups, (int)fsg_context::ROW_GROUPS)
                       : 1;
-    auto *ticket = (unsigned *)c->ensure(c->ticket, sizeof(unsigned) * G);
-    auto *bad = (int *)c->ensure(c->bad, sizeof(int) * nlos);
-    auto *nbad = (int *)c->ensure(c->nbad, sizeof(int));
-    auto *err = (unsigned *)c->ensure(c->err, sizeof(unsigned));
     cuda_check(cudaMemsetAsync(ticket, 0, sizeof(unsigned) * G, s), "memset");
     cuda_check(cudaMemsetAsync(nbad, 0, sizeof(int), s), "memset");
     cuda_check(cudaMemsetAsync(err, 0, sizeof(unsigned), s), "memset");
@@ -579,7 +611,7 @@ void deposit(fsg_context *c, const LineParams &lp, const Particles &p, double *o
         std::vector<long long> fill(start.begin(), start.end() - 1);
         for (int line : c->h_order)
             gord[(size_t)fill[group_of(line)]++] = line;
-        auto *dord = (int *)c->ensure(c->gorder, sizeof(int) * (size_t)nlos);
+        auto *dord = (int *)c->gorder.p;
         cuda_check(cudaMemcpyAsync(dord, gord.data(), sizeof(int) * (size_t)nlos,
                                    cudaMemcpyHostToDevice, s), "upload order");
         // the host vector must outlive the copy
@@ -803,16 +835,35 @@ fsg_tune_key tune_key(fsg_context *c, const LineParams &lp, int precision)
     return k;
 }
 
-// The grid of a configuration: resident CTAs on every SM, at most one per sightline.
+// The grid of a configuration: resident CTAs on every SM, at most one per sightline
+// unless they are shared.
+void set_grid(fsg_context *c, const LineParams &lp, DepositLaunch &cfg, int sms)
+{
+    const int per_sm = std::max(1, deposit_resident_ctas(cfg, lp.compute_tau, lp.nbins));
+    cfg.grid = cfg.split_ws ? sms * (cfg.split32 ? 1 : per_sm) : std::min(c->nlos, sms * per_sm);
+}
+
 void finish_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
 {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const int per_sm = std::max(1, deposit_resident_ctas(cfg, lp.compute_tau, lp.nbins));
     deposit_fit_chunk(cfg, c->npairs, sms);
     const size_t sb = deposit_split_bytes(cfg, lp.nbins, c->nlos, sms);
-    cfg.split_ws = sb ? c->ensure(c->split, sb) : nullptr;
-    cfg.grid = sb ? sms * (cfg.split32 ? 1 : per_sm) : std::min(c->nlos, sms * per_sm);
+    cfg.split_ws = sb ? c->ensure_split(sb) : nullptr;
+    set_grid(c, lp, cfg, sms);
+}
+
+// Once every buffer of the call is there: the shared-sightline buffer may have grown
+// since the plan named it, or have made room for another.
+void settle_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
+{
+    if (!cfg.split_ws)
+        return;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    const size_t sb = deposit_split_bytes(cfg, lp.nbins, c->nlos, sms);
+    cfg.split_ws = sb <= c->split.cap ? c->split.p : nullptr;
+    set_grid(c, lp, cfg, sms);
 }
 
 // Times the candidate launches on a sample of the call's sightlines (every
@@ -979,15 +1030,11 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
         p.dens = dens[k];
         apply_tuning(c, lps[k], opt, p, pl, outs[k], cfgs.back());
     }
-    // the forms differ in what they need: the shared-sightline buffer may have grown
-    // after an earlier deposit's plan named it, and any of them may accumulate in
-    // global memory
+    // the forms differ in what they need: any of them may accumulate in global memory
     bool global_acc = false;
     for (DepositLaunch &cf : cfgs) {
         if (cf.rec)
             pl.rec = c->ensure(c->prec, 32 * (size_t)c->npairs);
-        if (cf.split_ws)
-            cf.split_ws = c->split.p;
         global_acc = global_acc || !cf.smem_mode;
     }
     unsigned long long *gacc = nullptr;
@@ -997,6 +1044,8 @@ void run_batch(fsg_context *c, const std::vector<LineParams> &lps,
     auto *bad = (int *)c->ensure(c->bad, sizeof(int) * nlos);
     auto *nbad = (int *)c->ensure(c->nbad, sizeof(int));
     auto *err = (unsigned *)c->ensure(c->err, sizeof(unsigned));
+    for (size_t k = 0; k < lps.size(); k++)
+        settle_config(c, lps[k], cfgs[k]);
     // graph key: everything the captured launches depend on
     std::vector<double> key;
     auto put = [&](double v) { key.push_back(v); };
