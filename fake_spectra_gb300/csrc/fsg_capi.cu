@@ -731,7 +731,7 @@ DepositLaunch deposit_config(fsg_context *c, const LineParams &lp, const fsg_opt
 
 // ---------------------------------------------------------------- autotuner
 // The FP32 deposit's launch (threads per block, pairs staged per warp, queue
-// mode) is chosen by timing candidates on a sample of the call's own
+// mode; for shared sightlines the pairs staged per warp) is chosen by timing candidates on a sample of the call's own
 // sightlines, once per workload class (fsg_tune_key), and cached: in the
 // process, and in a text file when one is named (fsg_tune_cache_file or the
 // FSG_TUNE_CACHE environment variable).  Every candidate gives the same output
@@ -814,11 +814,14 @@ bool tune_store_locked(const fsg_tune_key &k, const fsg_tune_entry &e)
 
 int floor_log2x2(double v) { return (int)std::floor(2.0 * std::log2(v)); }
 
-fsg_tune_key tune_key(fsg_context *c, const LineParams &lp, int precision)
+// An FP32 optical depth whose sightlines are shared between blocks.
+bool shares32(const DepositLaunch &cfg) { return cfg.split32 && cfg.split_ws; }
+
+fsg_tune_key tune_key(fsg_context *c, const LineParams &lp, const DepositLaunch &cfg)
 {
     fsg_tune_key k{};
     cudaDeviceGetAttribute(&k.sms, cudaDevAttrMultiProcessorCount, c->device);
-    k.precision = precision;
+    k.precision = cfg.precision;
     k.compute_tau = lp.compute_tau;
     k.kernel = lp.kernel;
     k.nbins_b = floor_log2x2(std::max(1, lp.nbins));
@@ -831,6 +834,8 @@ fsg_tune_key tune_key(fsg_context *c, const LineParams &lp, int precision)
     k.pairs_med_b = floor_log2x2(1.0 + (double)q(0.5));
     k.pairs_p99_b = floor_log2x2(1.0 + (double)q(0.99));
     k.lines_b = (int)std::floor(std::log2((double)std::max(1, c->nlos)));
+    if (shares32(cfg))
+        k.lines_b = -1 - k.lines_b;
     k.damp_b = lp.compute_tau ? floor_log2x2(std::max(1e-300, lp.voigt_fac / lp.bfac)) : 0;
     return k;
 }
@@ -853,6 +858,17 @@ void finish_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
     set_grid(c, lp, cfg, sms);
 }
 
+// The launch that runs, in the statistics.
+void note_launch(fsg_context *c, const DepositLaunch &cfg, int tuned)
+{
+    const bool shared = shares32(cfg);
+    c->stats.launch_threads = shared ? split32_threads() : cfg.threads;
+    c->stats.launch_chunk = shared ? cfg.split32 : cfg.chunk;
+    c->stats.launch_persistent = shared ? 1 : cfg.persistent;
+    c->stats.launch_records = shared ? 0 : cfg.rec;
+    c->stats.launch_tuned = tuned;
+}
+
 // Once every buffer of the call is there: the shared-sightline buffer may have grown
 // since the plan named it, or have made room for another.
 void settle_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
@@ -864,17 +880,23 @@ void settle_config(fsg_context *c, const LineParams &lp, DepositLaunch &cfg)
     const size_t sb = deposit_split_bytes(cfg, lp.nbins, c->nlos, sms);
     cfg.split_ws = sb <= c->split.cap ? c->split.p : nullptr;
     set_grid(c, lp, cfg, sms);
+    if (!cfg.split_ws)
+        note_launch(c, cfg, 0);
 }
 
 // Times the candidate launches on a sample of the call's sightlines (every
 // k-th of the descending pair-count order, about four sightlines per resident
 // CTA so that the queue's balance resembles the full call's) and returns the
-// fastest.  The sample rows of `out` are overwritten.
+// fastest.  Shared sightlines (all of them in the sample) leave the pairs staged per
+// warp to choose.  The sample rows of `out` are overwritten.
 fsg_tune_entry tune_deposit(fsg_context *c, const LineParams &lp, const Particles &p,
                             PairLists pl, double *out, const DepositLaunch &base)
 {
     cudaStream_t s = c->stream;
     const int nlos = c->nlos;
+    const bool shared = shares32(base);
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     const int want = std::max(64, 4 * base.grid);
     const int nsamp = std::min(nlos, want);
     std::vector<int> order((size_t)nsamp);
@@ -895,7 +917,10 @@ fsg_tune_entry tune_deposit(fsg_context *c, const LineParams &lp, const Particle
         int threads, chunk, persistent, rec;
     };
     std::vector<Cand> cands;
-    if (lp.compute_tau)
+    if (shared)
+        cands = {{split32_threads(), 8, 1, 0}, {split32_threads(), 4, 1, 0},
+                 {split32_threads(), 2, 1, 0}};
+    else if (lp.compute_tau)
         cands = {{512, 8, 1, 0},  {512, 4, 1, 0},  {512, 16, 1, 0},  {512, 8, 0, 0},
                  {256, 8, 1, 0},  {768, 8, 1, 0},  {768, 16, 1, 0},  {1024, 4, 1, 0},
                  {1024, 8, 1, 0}, {1024, 16, 1, 0}, {1024, 8, 1, 1}, {768, 8, 1, 1}};
@@ -907,19 +932,22 @@ fsg_tune_entry tune_deposit(fsg_context *c, const LineParams &lp, const Particle
     best.sample_lines = nsamp;
     for (const Cand &cd : cands) {
         DepositLaunch cfg = base;
-        cfg.split_ws = nullptr;
-        cfg.threads = cd.threads;
-        cfg.chunk = cd.chunk;
-        cfg.persistent = cd.persistent;
-        cfg.rec = cd.rec;
-        cfg.tiles = base.tiles_asked;
-        deposit_plan(cfg, lp.compute_tau, lp.nbins);
-        if (cfg.smem_mode != base.smem_mode || cfg.tiles != base.tiles)
-            continue;   // only launches that keep the default's on-chip layout
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        const int per_sm = std::max(1, deposit_resident_ctas(cfg, lp.compute_tau, lp.nbins));
-        cfg.grid = std::min(nsamp, sms * per_sm);
+        if (shared) {
+            cfg.split32 = cd.chunk;
+            if (!deposit_split_bytes(cfg, lp.nbins, nlos, sms))
+                continue;
+        } else {
+            cfg.threads = cd.threads;
+            cfg.chunk = cd.chunk;
+            cfg.persistent = cd.persistent;
+            cfg.rec = cd.rec;
+            cfg.tiles = base.tiles_asked;
+            deposit_plan(cfg, lp.compute_tau, lp.nbins);
+            if (cfg.smem_mode != base.smem_mode || cfg.tiles != base.tiles)
+                continue;   // only launches that keep the default's on-chip layout
+            const int per_sm = std::max(1, deposit_resident_ctas(cfg, lp.compute_tau, lp.nbins));
+            cfg.grid = std::min(nsamp, sms * per_sm);
+        }
         pl.rec = cfg.rec ? c->ensure(c->prec, 32 * (size_t)c->npairs) : nullptr;
         float ms_min = 1e30f;
         for (int rep = 0; rep < 2; rep++) {
@@ -937,8 +965,9 @@ fsg_tune_entry tune_deposit(fsg_context *c, const LineParams &lp, const Particle
             ms_min = std::min(ms_min, ms);
         }
         best.candidates++;
-        if (cd.threads == base.threads && cd.chunk == base.chunk &&
-            cd.persistent == base.persistent && cd.rec == base.rec)
+        if (shared ? cd.chunk == base.split32
+                   : cd.threads == base.threads && cd.chunk == base.chunk &&
+                         cd.persistent == base.persistent && cd.rec == base.rec)
             best.ms_default = ms_min;
         if (ms_min < best.ms_best) {
             best.ms_best = ms_min;
@@ -961,17 +990,14 @@ fsg_tune_entry tune_deposit(fsg_context *c, const LineParams &lp, const Particle
 void apply_tuning(fsg_context *c, const LineParams &lp, const fsg_options *opt, const Particles &p,
                   PairLists pl, double *out, DepositLaunch &cfg)
 {
-    c->stats.launch_threads = cfg.threads;
-    c->stats.launch_chunk = cfg.chunk;
-    c->stats.launch_persistent = cfg.persistent;
-    c->stats.launch_records = cfg.rec;
-    c->stats.launch_tuned = 0;
+    note_launch(c, cfg, 0);
     const int mode = opt ? opt->tune : 0;
     if (cfg.precision != FSG_PREC_FP32 || lp.kernel == VORONOI || mode < 0 || !opt ||
         opt->count_work || opt->threads > 0 || opt->chunk > 0 || opt->persistent >= 0 ||
         opt->records >= 0 || c->nlos <= 0 || pl.seg)
         return;
-    const fsg_tune_key key = tune_key(c, lp, cfg.precision);
+    const fsg_tune_key key = tune_key(c, lp, cfg);
+    const bool shared = shares32(cfg);
     fsg_tune_entry e{};
     bool have = false;
     {
@@ -984,6 +1010,17 @@ void apply_tuning(fsg_context *c, const LineParams &lp, const fsg_options *opt, 
         }
     }
     if (!have) {
+        if (shared) {
+            // the timing's buffers first: they may need the shared sightlines' room
+            c->ensure(c->tune_order, sizeof(int) * (size_t)c->nlos);
+            c->ensure(c->ticket, sizeof(unsigned));
+            c->ensure(c->bad, sizeof(int) * c->nlos);
+            c->ensure(c->nbad, sizeof(int));
+            c->ensure(c->err, sizeof(unsigned));
+            settle_config(c, lp, cfg);
+            if (!cfg.split_ws)
+                return;
+        }
         e = tune_deposit(c, lp, p, pl, out, cfg);
         c->stats.tune_ran = 1;
         c->stats.tune_candidates = e.candidates;
@@ -994,6 +1031,16 @@ void apply_tuning(fsg_context *c, const LineParams &lp, const fsg_options *opt, 
         tune_store_locked(key, e);
     }
     DepositLaunch t = cfg;
+    if (shared) {
+        t.split32 = e.chunk;
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        if (e.threads != split32_threads() || !deposit_split_bytes(t, lp.nbins, c->nlos, sms))
+            return;
+        cfg = t;
+        note_launch(c, cfg, 1);
+        return;
+    }
     t.threads = e.threads;
     t.chunk = e.chunk;
     t.persistent = e.persistent;
@@ -1004,11 +1051,7 @@ void apply_tuning(fsg_context *c, const LineParams &lp, const fsg_options *opt, 
         return;   // a cached choice that does not fit this call's layout
     finish_config(c, lp, t);
     cfg = t;
-    c->stats.launch_threads = cfg.threads;
-    c->stats.launch_chunk = cfg.chunk;
-    c->stats.launch_persistent = cfg.persistent;
-    c->stats.launch_records = cfg.rec;
-    c->stats.launch_tuned = 1;
+    note_launch(c, cfg, 1);
 }
 
 // The batched form (fsg_spectra_batch_device): every deposit of the call in

@@ -3250,6 +3250,8 @@ int fast64_resident(int compute_tau, int threads, size_t smem)
 }
 }  // namespace
 
+int split32_threads() { return SPLIT32_THREADS; }
+
 int fast64_threads(int compute_tau) { return compute_tau ? T64_THREADS : C64_THREADS; }
 
 // Smaller chunks for small calls: at least four per warp of the whole device

@@ -334,6 +334,7 @@ size_t deposit_smem_bytes(const DepositLaunch &cfg, int compute_tau, int nbins);
 // makes the planned chunks small enough for a call of npairs pairs.
 int fast64_threads(int compute_tau);   // default block size
 void deposit_fit_chunk(DepositLaunch &cfg, long long npairs, int sms);
+int split32_threads();                 // block size of shared FP32 optical depths
 size_t deposit_split_bytes(const DepositLaunch &cfg, int nbins, int nlos, int sms);
 // CTAs of the deposit kernel that fit on one SM for this configuration.
 int deposit_resident_ctas(const DepositLaunch &cfg, int compute_tau, int nbins);

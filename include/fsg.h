@@ -328,7 +328,8 @@ typedef struct {
     int32_t nbins_b;      /* floor(2 log2 nbins)                                 */
     int32_t pairs_med_b;  /* floor(2 log2(1 + median pairs per sightline))      */
     int32_t pairs_p99_b;  /* floor(2 log2(1 + 99th-percentile pairs per line))  */
-    int32_t lines_b;      /* floor(log2 sightlines)                              */
+    int32_t lines_b;      /* floor(log2 sightlines); -1 - that where an FP32 optical
+                             depth's sightlines are shared between blocks        */
     int32_t damp_b;       /* floor(2 log2(Gamma lambda / 4 pi / b(T = 1 K)))    */
 } fsg_tune_key;
 
