@@ -1661,20 +1661,20 @@ __device__ const TileTables g_tile = tile_tables();
 // for A_r >= 0, so Newton's method from W0 = tautail / A_0 (h(W0) >= tautail)
 // decreases monotonically to the root.  Returns +inf when tautail <= 0 (the
 // window then runs to the cap) and 0 when the wing is identically zero.
-__device__ __forceinline__ float far_stop_radius(const Tau32 &s, float tautail)
+__device__ __forceinline__ float far_stop_radius(const float (&A)[MP_R], float tautail)
 {
     if (!(tautail > 0.f))
         return __int_as_float(0x7f800000);
-    if (!(s.A[0] > 0.f))
+    if (!(A[0] > 0.f))
         return 0.f;
-    float W = tautail / s.A[0];
+    float W = tautail / A[0];
 #pragma unroll 1
     for (int it = 0; it < 4; it++) {
-        float h = s.A[MP_R - 1], d = (float)MP_R * s.A[MP_R - 1];
+        float h = A[MP_R - 1], d = (float)MP_R * A[MP_R - 1];
 #pragma unroll
         for (int r = MP_R - 2; r >= 0; r--) {
-            h = fmaf(h, W, s.A[r]);
-            d = fmaf(d, W, (float)(r + 1) * s.A[r]);
+            h = fmaf(h, W, A[r]);
+            d = fmaf(d, W, (float)(r + 1) * A[r]);
         }
         W -= (h * W - tautail) / d;
     }
@@ -1719,7 +1719,7 @@ __device__ __forceinline__ void walk_tau32_tiled(const DepositArgs &a, const Tau
                                              : (jb + 1) % TILE_W;
                     if (rem == 0) {
                         if (vsure < 0.f)
-                            vsure = 0.999f * far_stop_radius(s, tautail);
+                            vsure = 0.999f * far_stop_radius(s.A, tautail);
                         const float klim = dir == 0 ? (vsure - s.vmid0) / s.vk
                                                     : (vsure + s.vmid0) / s.vk - 1.f;
                         n = 0;
@@ -2794,9 +2794,15 @@ __device__ __forceinline__ GradSums grad_far(const StageGrad &g, float V)
 // pair's window (every lane holds its part afterwards).  The walk is the
 // forward's: pixel steps, and where the forward deposits through the nodes of
 // far-field tiles, the transpose of that, the pair's value at each node times
-// the node's share of dL/dtau (grow: the row's pixels, gnode: its nodes; gnode
-// null: every pixel).  128^3, 1024 sightlines x 1115 pixels: 8.66 ms with all
-// seven nodes at every pixel of the window, 5.3 ms so.
+// the node's share of dL/dtau (grow: the row's pixels, gnode: its nodes).
+// 128^3, 1024 sightlines x 1115 pixels: 8.66 ms with all seven nodes at every
+// pixel of the window, 5.05 ms so.
+// Bound by instruction issue and, for windows of a few steps, by the instruction
+// cache and spills at 64 registers: with the tiles' state live through the pixel
+// steps, and a vote per sample, Ly-b rows of 650 to 800 pixels took 1.20 times
+// the seven-node walk's 1.33 ms, now 1.11 times, less than the forward gained.
+// A second walk for such pairs beside this one (inlined or called) is slower on
+// every row: the warps of a block then run two copies of the node sums.
 __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, const float *grow,
                                             const float *gnode, int nbins, float tautail,
                                             int lane, const float2 *vtab, float &ad, float &av,
@@ -2809,98 +2815,92 @@ __device__ __forceinline__ void grad_pair32(const StageGrad &g, const Tau32 &s, 
     ad = av = at = 0.f;
     for (int dir = 0; dir < 2; dir++) {
         // the distance from which tiles are tried (infinite: no more)
-        float dmin = s.tiles && gnode != nullptr ? fmaxf(s.vmp, TILE_DIST * s.vk) : INFINITY;
-        int k = 0, items = 0, base = 0, jb_run = 0;
+        float dmin = s.tiles ? fmaxf(s.vmp, TILE_DIST * s.bintov * s.inv_b) : INFINITY;
+        int k = 0;
         while (k < half) {
-            const int koff0 = dir == 0 ? k : -1 - k;
-            const float kf0 = (float)koff0;
+            const float kf0 = (float)(dir == 0 ? k : -1 - k);
             int len = 32;
-            if (items == 0 &&
-                (dir == 0 ? fmaf(kf0, s.vk, s.v0) : -fmaf(kf0 + 1.f, s.vk, s.v0)) >= dmin) {
-                const int jb = bin_from(j0, koff0, nbins);
+            const float d0 = fmaf(dir == 0 ? kf0 : kf0 + 1.f, s.bintov, s.base0) * s.inv_b;
+            if ((dir == 0 ? d0 : -d0) >= dmin) {
+                // (formed here, and the tiles' run a loop of its own: kept live through
+                // the pixel steps they spilled)
+                const float vk = s.bintov * s.inv_b, v0 = s.base0 * s.inv_b,
+                            vmid0 = v0 + s.hbin_b;
+                const int jb = bin_from(j0, dir == 0 ? k : -1 - k, nbins);
                 const int rem = dir == 0 ? (TILE_W - jb % TILE_W) % TILE_W : (jb + 1) % TILE_W;
                 // the next tile is inside the window when its last pixel's value, taken
                 // 0.11% farther out, is above tautail
                 const float kt = (float)(k + rem) + (float)(TILE_W - 1);
-                const float ve = dir == 0 ? fmaf(kt, s.vk, s.vmid0)
-                                          : fmaf(kt + 1.f, s.vk, -s.vmid0);
+                const float ve = dir == 0 ? fmaf(kt, vk, vmid0) : fmaf(kt + 1.f, vk, -vmid0);
                 if (half - k - rem < TILE_W ||
                     !(s.scale * grad_far(g, 1.0011f * ve).d >= tautail)) {
                     dmin = INFINITY;       // the window ends before the next tile does
                 } else if (rem == 0) {
-                    const float vsure = 0.999f * far_stop_radius(s, tautail);
-                    const float klim = dir == 0 ? (vsure - s.vmid0) / s.vk
-                                                : (vsure + s.vmid0) / s.vk - 1.f;
+                    const float vsure = 0.999f * far_stop_radius(g.s.A, tautail / s.scale);
+                    const float klim = dir == 0 ? (vsure - vmid0) / vk
+                                                : (vsure + vmid0) / vk - 1.f;
                     int n = (int)fminf((klim - (float)k + 1.f) / (float)TILE_W, 1e6f);
                     n = min(n, (half - k) / TILE_W);
                     n = min(n, dir == 0 ? (nbins - jb) / TILE_W : (jb + 1) / TILE_W);
                     if (n > 0) {
-                        items = n * TILE_M;
-                        base = 0;
-                        jb_run = jb;
-                    } else if (dir != 0 || nbins - jb >= TILE_W) {
-                        dmin = INFINITY;
+                        // a run of tiles: the value at each node (the wing's) times the
+                        // node's share of dL/dtau
+                        const int items = n * TILE_M;
+                        for (int it = lane; it < items; it += 32) {
+                            const int t = it / TILE_M, m = it - t * TILE_M;
+                            const int k0 = k + TILE_W * t;
+                            const float x =
+                                fmaf(g_tile.x[m], vk,
+                                     fmaf((float)(dir == 0 ? k0 : -k0 - TILE_W), vk, v0));
+                            const int j = dir == 0 ? jb + TILE_W * t : jb - TILE_W * (t + 1) + 1;
+                            const float gg = gnode[j / TILE_W * TILE_M + m];
+                            for (int i = 0; i < np; i++) {
+                                const float xi = np == 1 ? x + s.hbin_b
+                                                 : i == np - 1 ? fmaf(2.f, s.hbin_b, x)
+                                                               : fmaf((float)i, s.sub_dv, x);
+                                const GradSums h = grad_far(g, xi);
+                                const float wt =
+                                    np > 1 && (i == 0 || i == np - 1) ? 0.5f * gg : gg;
+                                ad = fmaf(wt, h.d, ad);
+                                av = fmaf(wt, h.v, av);
+                                at = fmaf(wt, h.t, at);
+                            }
+                        }
+                        __syncwarp();
+                        k += TILE_W * n;
+                        continue;
                     }
+                    if (dir != 0 || nbins - jb >= TILE_W)
+                        dmin = INFINITY;
                 } else {
                     len = min(32, rem);
                 }
             }
-            // one evaluation per lane: a tile node or a pixel; the position is x mul
-            // (mul: to units of b) plus the sample's offset
-            float x, mul = 1.f;
-            if (items) {
-                const int it = min(base + lane, items - 1);
-                const int t = it / TILE_M, m = it - t * TILE_M;
-                const int kt = k + TILE_W * t;
-                x = fmaf((float)(dir == 0 ? kt : -kt - TILE_W), s.vk, s.v0);
-                x = fmaf(g_tile.x[m], s.vk, x);
-            } else {
-                x = fmaf(dir == 0 ? kf0 + lane_f : kf0 - lane_f, s.bintov, s.base0);
-                mul = s.inv_b;
-            }
+            const float x = fmaf(dir == 0 ? kf0 + lane_f : kf0 - lane_f, s.bintov, s.base0);
             // The stop rule compares with tautail: where the wing polynomial comes
             // within 1e-4 of it (its own error is 1e-6) the node sums decide.  A stop
             // one pixel off moves the temperature gradient of a weak particle, whose
             // window ends on its Gaussian flank, by 1e-3 of the largest.
             GradSums r;
-            bool nodes = false;
-            do {
-                bool poly = false;
+            // every sample of every lane beyond vmp (the samples are within half a pixel)
+            const float mid = fabsf(fmaf(x, s.inv_b, s.hbin_b));
+            bool wing = __all_sync(0xffffffffu, mid - (np == 1 ? 0.f : s.hbin_b) >= s.vmp);
+            for (;;) {
                 r = {0.f, 0.f, 0.f};
                 for (int i = 0; i < np; i++) {
-                    const float xi = np == 1 ? fmaf(x, mul, s.hbin_b)
-                                     : i == np - 1 ? fmaf(x, mul, 2.f * s.hbin_b)
-                                                   : fmaf((float)i, s.sub_dv, __fmul_rn(x, mul));
-                    const bool wing = !nodes && __all_sync(0xffffffffu, fabsf(xi) >= s.vmp);
+                    const float xi = np == 1 ? fmaf(x, s.inv_b, s.hbin_b)
+                                     : i == np - 1 ? fmaf(x, s.inv_b, 2.f * s.hbin_b)
+                                                   : fmaf((float)i, s.sub_dv, __fmul_rn(x, s.inv_b));
                     const GradSums h = wing ? grad_far(g, xi) : grad_node_sums(s, xi, vtab);
                     const float wt = np > 1 && (i == 0 || i == np - 1) ? 0.5f : 1.f;
                     r.d = fmaf(wt, h.d, r.d);
                     r.v = fmaf(wt, h.v, r.v);
                     r.t = fmaf(wt, h.t, r.t);
-                    poly |= wing;
                 }
-                nodes = poly && !items &&
-                        __any_sync(0xffffffffu, fabsf(fmaf(s.scale, r.d, -tautail)) <=
-                                                    1e-4f * tautail);
-            } while (nodes);
-            // times dL/dtau of the pixel, or the node's share of it
-            if (items) {
-                const int it = base + lane;
-                if (it < items) {
-                    const int t = it / TILE_M;
-                    const float gg = gnode[(dir == 0 ? jb_run + TILE_W * t
-                                                     : jb_run - TILE_W * (t + 1) + 1) / TILE_W *
-                                               TILE_M + it - t * TILE_M];
-                    ad = fmaf(gg, r.d, ad);
-                    av = fmaf(gg, r.v, av);
-                    at = fmaf(gg, r.t, at);
-                }
-                base += 32;
-                if (base >= items) {
-                    k += TILE_W * (items / TILE_M);
-                    items = 0;
-                }
-                continue;
+                if (!wing || !__any_sync(0xffffffffu, fabsf(fmaf(s.scale, r.d, -tautail)) <=
+                                                          1e-4f * tautail))
+                    break;
+                wing = false;
             }
             const int kk = k + lane;
             bool on = lane < len && kk < half;
