@@ -3053,8 +3053,6 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(GradArgs a)
 
 int g_max_smem_optin = -1;
 
-// The kernel build for a block size: the FP32 tau form (not counting) has
-// 768- and 1024-thread builds beside the default.
 // The kernel build for a block size and input path: the FP32 optical-depth
 // deposit has 512-, 768- and 1024-thread builds, each gathering the particle
 // fields or reading pair records; the FP32 column density has 512- and
@@ -3114,8 +3112,20 @@ int max_smem_optin()
     }
     return g_max_smem_optin;
 }
-// static shared memory of the deposit kernel is < 1.5 KiB
+// Kept free of dynamic shared memory in every plan: the kernels' static arrays (the
+// records build of deposit_kernel has 1736 bytes, the FP64 optical depth 1544) and a
+// few scalars.
 constexpr int STATIC_SMEM_RESERVE = 2048;
+constexpr size_t STATIC_SCALARS = 128;
+static_assert(sizeof(BoundScratch) + sizeof(float2) * FSG_V32_N + sizeof s_stage_bar +
+                      sizeof s_stage_phase + STATIC_SCALARS <= STATIC_SMEM_RESERVE,
+              "deposit_kernel, split32_kernel and grad_kernel fit the reserve");
+static_assert(sizeof(BoundScratch) + sizeof s_cos64 + sizeof s_node64 + sizeof s_pow2 +
+                      STATIC_SCALARS <= STATIC_SMEM_RESERVE,
+              "fast64_kernel fits the reserve");
+static_assert(sizeof(BoundScratch) + (sizeof(int) + sizeof(double)) * MAX_CHANNELS +
+                      STATIC_SCALARS <= STATIC_SMEM_RESERVE,
+              "colden_channels_kernel fits the reserve");
 }  // namespace
 
 namespace {
