@@ -94,7 +94,7 @@ struct fsg_context {
     DevBuf flag, tcount, tstart, tsums, idx;                 // _near_lines
     DevBuf fpart, fout, fedges, fcounts, ftau, fdflux, ffft, fpower;   // flux statistics
     DevBuf ptables, pchirp, pbhat, pfused, ppart;            // flux power plan and partials
-    DevBuf fexp;                                             // 2^(j/256) of the flux exponential
+    DevBuf fexp;                                             // 2^(-k/1024) of the flux exponential
     bool fexp_ready = false;
     PowerPlan pplan;                                         // plan of the last flux power call
     DevBuf vseg, vscratch, vcofm;                            // Voronoi cells

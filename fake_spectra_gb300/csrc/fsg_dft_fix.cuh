@@ -8,10 +8,10 @@
 // once.
 //
 // Scaling.  By Cauchy's inequality no value of a partial transform that combines
-// m inputs exceeds sqrt(m) |z|_2.  The input is scaled so that |z|_2 <= 2^60 and
+// m inputs exceeds sqrt(m) |z|_2.  The input is scaled so that |z|_2 <= 2^60.8 and
 // each pass divides by a power of two so that what m inputs have been combined
-// into is divided by sqrt(m) at least: every stored value stays below 2^60 and,
-// inside a pass of radix R <= 16, below sqrt(R) 2^60.  A typical value is
+// into is divided by sqrt(m) at least: every stored modulus stays below 2^60.8 and,
+// inside a pass of radix R <= 16, below sqrt(R) 2^60.8 <= 2^62.8.  A typical value is
 // 2^60 / sqrt(m), so for transforms of 1e4 points values keep 53 bits and the
 // rounding of all passes together stays below that of FP64 arithmetic.
 //
@@ -56,10 +56,12 @@ FSG_HD FixSplit fix_split(int64_t a)
     return {(int32_t)((a - lo) >> 32), lo};
 }
 
-// a w / 2^e, e = 0, 1 or 2, rounded, ties up or (odd = 1) down: a factor of 1 meets
-// ties, and values of one column rounded the same way would add up.  |a| <= 2^62
-// keeps the sums of products below 2^63 (|lo| <= 2^31, |c|, |s| hi <= 2^30, and by
-// modulus each pair of products below sqrt(2) times its larger bound).
+// a w / 2^e, e = 1 or 2, rounded, ties up or (odd = 1) down: a factor of 1 meets
+// ties, and values of one column rounded the same way would add up.  A modulus of a
+// up to 2^62.8 keeps the sums below 2^63: the products of a's low words (at most 2^31
+// each) with w's high words (modulus 2^30) are below 2^61.5 together, those of a's high
+// words (modulus 2^30.8) with w's low words below 2^62.3, those of the high words
+// below 2^60.8 (2^61.8 shifted).
 FSG_HD FixC fixc_mul(FixC a, FixW w, int e, int odd)
 {
     const FixSplit x = fix_split(a.x), y = fix_split(a.y);
@@ -356,7 +358,7 @@ FSG_HD void filter_butterfly(FixC *x, const FixW *w, unsigned f, unsigned L, int
         p[r] = v[r];
 }
 
-// d in units of 2^-sh, rounded (|d| < 2^(62 - sh); d = 0 below 2^-1022)
+// d in units of 2^-sh, rounded (|d| < 2^(63 - sh); d = 0 below 2^-1022)
 FSG_HD int64_t fix_from_double(double d, int sh)
 {
 #ifdef __CUDA_ARCH__

@@ -428,11 +428,11 @@ __device__ __forceinline__ void warp_for_each_pair(const LineTables &t, const fl
     }
 }
 
-// Lanes that meet the same sightline together share one atomic. (the particles
-// of a warp are spatial neighbours once sorted, so they often do).
+// Lanes that meet the same sightline together share one atomic (the particles of a
+// warp are spatial neighbours once sorted, so they often do).
 __global__ void __launch_bounds__(256, 4)
     count_pairs_kernel(LineTables t, Particles p, const int *perm,
-                                   unsigned long long *line_count, unsigned char *part_flag)
+                       unsigned long long *line_count, unsigned char *part_flag)
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(256, 4)
 
 __global__ void __launch_bounds__(256, 4)
     emit_pairs_kernel(LineTables t, Particles p, const int *perm, const long long *off,
-                                  unsigned long long *cursor, int *part, unsigned *dev_err)
+                      unsigned long long *cursor, int *part, unsigned *dev_err)
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
