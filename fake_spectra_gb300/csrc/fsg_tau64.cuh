@@ -516,7 +516,11 @@ __device__ __forceinline__ void walk_tau64(const DepositArgs &a, const Tiles64 &
     const bool tiles = w0 > 0 && (st.flags & S64_TILES);
     int kmp = 0, ksure = 0;
     if (tiles) {
-        kmp = (int)fminf(st.vmp / st.vk * 1.00001f + 2.f, 1e9f);
+        // one pixel for the centre's place in its own, up to half a pixel for the first
+        // sample of the pixel about the first node: every sample of every node is
+        // beyond vmp, so tiles never take the node sums, whose range ends a step of 32
+        // pixels beyond it
+        kmp = (int)fminf(st.vmp / st.vk * 1.00001f + 3.f, 1e9f);
         ksure = (int)fminf(st.vsure / st.vk - 2.f, 1e9f);
     }
     const int np = st.flags & S64_NP;
@@ -584,9 +588,9 @@ __device__ __forceinline__ void walk_tau64(const DepositArgs &a, const Tiles64 &
             int idx = 0;
             bool on;
             if (items > 0) {
-                const int it = base + lane;
-                on = it < items;
-                int t = on ? it / T64_M : 0;
+                on = base + lane < items;
+                const int it = min(base + lane, items - 1);
+                int t = it / T64_M;
                 const int m = it % T64_M;
                 int l = 0, ct = rc[0];
                 bool found = false;
