@@ -1210,7 +1210,7 @@ __device__ __forceinline__ double colden_pair_bound(const LineParams &lp, const 
 // would not be, and the kernels without a square root keep the double form.
 struct ColdenEnds {
     bool fix, cubic;
-    double inv_h;            // 2^62 / h
+    double inv_h;            // fix_spline_scale
     uint64_t B;              // dr2 / h^2, units of 2^-64
     __device__ __forceinline__ explicit ColdenEnds(const Colden &c)
     {
@@ -1219,7 +1219,7 @@ struct ColdenEnds {
         fix = (cubic || c.kernel == SPH_QUINTIC) && c.zrange * c.zrange * 4096.0 > h2 &&
               h2 < 1e200 && h2 > 1e-200 && c.zrange <= c.smooth;
         const double inv = 1.0 / c.smooth;
-        inv_h = 4611686018427387904.0 * inv;
+        inv_h = fix_spline_scale(inv, c.smooth, c.zrange);
         B = fix ? __double2ull_rn(c.dr2 * inv * inv * 18446744073709551616.0) : 0ull;
     }
     __device__ __forceinline__ double value(const Colden &c, long long z) const

@@ -48,26 +48,25 @@ def test_clipped_pixels(tmp_path, cubic, h):
         zr = float(np.sqrt(np.float64(np.float32(h) * np.float32(h)) - dr2))
         if zr > h:
             continue
-        cases += [(dr2, -zr, zr), (dr2, -zr, -zr), (dr2, zr, zr)]
+        cases += [(dr2, zr, -zr, zr), (dr2, zr, -zr, -zr), (dr2, zr, zr, zr)]
         for w in (1e-12, 1e-7, 1e-3, 0.1, 0.3, 0.9, 1.0, 1.5, 1.99):
             for f in (1.0, rng.random()):
                 d = min(w * f * zr, 2 * zr)
-                cases += [(dr2, -zr, -zr + d), (dr2, zr - d, zr)]
-    text = "\n".join("%d %s %s %s %s" % (cubic, h.hex(), a.hex(), b.hex(), c.hex())
-                     for a, b, c in cases)
+                cases += [(dr2, zr, -zr, -zr + d), (dr2, zr, zr - d, zr)]
+    text = "\n".join(" ".join([str(cubic), h.hex()] + [v.hex() for v in c]) for c in cases)
     out = subprocess.run([exe], input=text, capture_output=True, text=True, check=True).stdout
     got = [float.fromhex(s) for s in out.split()]
     assert len(got) == len(cases)
-    for (dr2, a, b), g in zip(cases, got):
+    for (dr2, _, a, b), g in zip(cases, got):
         want = tol = LD(0)
         for j in range(9):
             z = (LD(a) + (LD(b) - LD(a)) * j / 8) / LD(h)
             q = np.sqrt(LD(dr2) / LD(h) / LD(h) + z * z)
             k, dk = _kernel(cubic, q)
-            # z / h and dr2 / h^2 in double are good to 2^-51 of q (the derivative where
-            # q is that much smaller); the squares to 2^-63, the root to 2^-61 and
-            # every product to a unit of 2^-59
-            dq = LD(2) ** -50
+            # z / h and dr2 / h^2 in double are good to 2^-51 of q, and to 2^-49 where the
+            # scale is 8 units lower (the derivative where q is that much smaller); the
+            # squares to 2^-63, the root to 2^-61 and every product to a unit of 2^-59
+            dq = LD(2) ** (-50 if dr2 > 1e-14 * h * h else -48)
             dk = max(dk, _kernel(cubic, max(q - dq, LD(0)))[1])
             c = LD(1) / 2 if j in (0, 8) else LD(1)
             want += c * k
